@@ -158,6 +158,35 @@ __device__ __forceinline__ void reset_counter(unsigned int *counter) {
   if (t == 0) *counter = 0u;
 }
 
+/* tile t of nt along x, then y, then z (32-bit division whenever nt fits) */
+__device__ __forceinline__ void tile_of(unsigned long long t, unsigned long long nt, unsigned tx,
+                                        unsigned ty, unsigned &bx, unsigned &by, unsigned &bz) {
+  unsigned long long r = nt >> 32 ? t / tx : (unsigned long long)((unsigned)t / tx);
+  bx = (unsigned)(t - r * tx);
+  bz = nt >> 32 ? (unsigned)(r / ty) : (unsigned)r / ty;
+  by = (unsigned)(r - (unsigned long long)bz * ty);
+}
+
+/* CTAs of `threads` threads of a kernel without dynamic shared memory that
+ * one SM holds at a time, at least 1 (asked of CUDA once per kernel and CTA
+ * size: the answer is a constant of the device the process runs on) */
+inline int resident_ctas(const void *kern, int threads) {
+  struct Known { const void *k; int t, n; };
+  static thread_local Known known[64];
+  Known &e = known[((size_t)kern / 16 + (size_t)threads / 32 * 7) % 64];
+  if (e.k != kern || e.t != threads) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, 0) != cudaSuccess) {
+      (void)cudaGetLastError();
+      n = 1;
+    }
+    e.k = kern;
+    e.t = threads;
+    e.n = n > 0 ? n : 1;
+  }
+  return e.n;
+}
+
 /* CTA tile of the temporal-blocking kernels (ob2_tblock, ops_b200_loop.h) */
 #ifndef OB2_TB_TX
 #define OB2_TB_TX 64

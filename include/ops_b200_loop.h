@@ -115,9 +115,8 @@ typedef struct ob2_loop {
   void *ev_start, *ev_end;  /* timing events (diagnostics level > 1) */
   double host_t0;
   int block[3];             /* suggested CTA shape */
-  int grid[3];              /* suggested grid: x covers the range, y/z capped
-                               at about one full wave of resident CTAs; the
-                               kernel loops over the remaining y/z */
+  int grid[3];              /* suggested grid: one thread per point (loops with
+                               reductions: see ob2_red_grid) */
   int idx32;                /* 1: every dat has < 2^31 elements, so element
                                offsets fit 32-bit arithmetic */
   int tune;                 /* >= 0: this launch times block-shape candidate
@@ -192,6 +191,14 @@ OPS_API void ob2_flush(void);
 OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int dim,
                            const int *range, ops_arg *args, int nargs);
 OPS_API void ob2_loop_end(ob2_loop *L);
+/* Grid of a reduction loop whose threads take up to max_rows consecutive
+ * rows of a tile: *rows = max_rows when tiles of that height fill a wave of
+ * CTAs (`resident` per SM, times OPS_B200_RED_WAVES), else 1; tiles[0..2] =
+ * tiles of L->block along x, y (block[1] * rows rows) and z (the folded 3rd
+ * to 5th axes).  Returns the CTAs: one wave at most, evened out over the
+ * trips; L->partials is made large enough for them. */
+OPS_API unsigned ob2_red_grid(ob2_loop *L, int max_rows, int resident, unsigned tiles[3],
+                              int *rows);
 /* 1 when some dat is passed more than once and written through one of the
  * arguments: the loop's kernel must then not assume its dat pointers are
  * unaliased. */

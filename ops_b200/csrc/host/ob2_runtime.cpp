@@ -121,6 +121,7 @@ struct Runtime {
   std::vector<KStat> kstats;
   std::unordered_map<std::string, int> kindex;
   int block_x = 32, block_y = 4, block_z = 1;
+  bool block_set = false;  // the CTA shape was given by the user
   int device = 0;
   int sms = 148;
   // reduction scratch: per-CTA partials + finish counter
@@ -1542,9 +1543,9 @@ OPS_API void ops_init(const int argc, const char *const argv[], const int diags)
     const char *a = argv[i];
     const char *p;
     if ((p = strstr(a, "-OPS_DIAGS="))) I().OPS_diags = atoi(p + 11);
-    if ((p = strstr(a, "OPS_BLOCK_SIZE_X="))) r.block_x = atoi(p + 17);
-    if ((p = strstr(a, "OPS_BLOCK_SIZE_Y="))) r.block_y = atoi(p + 17);
-    if ((p = strstr(a, "OPS_BLOCK_SIZE_Z="))) r.block_z = atoi(p + 17);
+    if ((p = strstr(a, "OPS_BLOCK_SIZE_X="))) r.block_x = atoi(p + 17), r.block_set = true;
+    if ((p = strstr(a, "OPS_BLOCK_SIZE_Y="))) r.block_y = atoi(p + 17), r.block_set = true;
+    if ((p = strstr(a, "OPS_BLOCK_SIZE_Z="))) r.block_z = atoi(p + 17), r.block_set = true;
     if ((p = strstr(a, "OPS_DEVICE="))) r.device = atoi(p + 11);
     // loop-chain tiling (ops_lib_core.cpp:132-180): lazy queue + tiles
     if (strstr(a, "OPS_TILING")) r.lazy = r.tiling = true;
@@ -1590,7 +1591,9 @@ OPS_API void ops_init(const int argc, const char *const argv[], const int diags)
   if ((e = getenv("OPS_B200_DEVICE"))) r.device = atoi(e);
   else if ((e = getenv("OPS_B200_DIST")) && !strcmp(e, "nccl") && getenv("LOCAL_RANK"))
     r.device = atoi(getenv("LOCAL_RANK"));  // one process per GPU
-  if ((e = getenv("OPS_B200_BLOCK"))) sscanf(e, "%d,%d,%d", &r.block_x, &r.block_y, &r.block_z);
+  if ((e = getenv("OPS_B200_BLOCK")) &&
+      sscanf(e, "%d,%d,%d", &r.block_x, &r.block_y, &r.block_z) > 0)
+    r.block_set = true;
   if (r.block_x < 1) r.block_x = 32;
   if (r.block_y < 1) r.block_y = 1;
   if (r.block_z < 1) r.block_z = 1;
@@ -2349,6 +2352,16 @@ OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int d
   L->block[0] = r.block_x;
   L->block[1] = dim > 1 ? r.block_y : 1;
   L->block[2] = dim > 2 ? r.block_z : 1;
+  // reductions under the default shape: 256 threads, half as many per-CTA
+  // partials and tickets (the last CTA combines them) as 128
+  bool reduces = false;
+  for (int i = 0; i < nargs; i++)
+    if (args[i].argtype == OPS_ARG_GBL && args[i].acc != OPS_READ) reduces = true;
+  if (reduces && !r.block_set) {
+    L->block[0] = dim > 1 ? 32 : 256;
+    L->block[1] = dim > 1 ? 8 : 1;
+    L->block[2] = 1;
+  }
   L->host_t0 = wall();
   L->ev_start = L->ev_end = nullptr;
   L->fuse_id = -1;  // the stub names its fused launcher after this call
@@ -2359,7 +2372,6 @@ OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int d
   L->tb_role = nullptr;
   if (L->npoints == 0) return 0;
 
-  size_t red_bytes = 0;
   int nred = 0;
   L->idx32 = 1;
   const int soa = I().OPS_soa;
@@ -2463,29 +2475,15 @@ OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int d
       L->red[i].first = x.pending_first;
       L->red[i].op = a.acc;
       x.pending_first = 0;
-      red_bytes += (size_t)h->size;
       nred++;
     }
   }
-  // scratch for per-CTA partials (grid = ceil(n/block) per axis); each
-  // reduction argument's region is rounded up to 256 bytes by the stub
-  // grid: x covers the range; y and z are capped so that the grid is about
-  // one wave of resident CTAs (SMs x CTAs per SM), threads loop over the rest
   L->tune = -1;
   if (r.autotune && nred == 0 && dim >= 2 && dim <= 3) tune_pick(L);
   {
-    long long tpb = (long long)L->block[0] * L->block[1] * L->block[2];
-    long long per_sm = std::max(1LL, 2048 / tpb);
-    long long target = (long long)r.sms * per_sm * r.red_waves;
     long long gx = (L->n[0] + L->block[0] - 1) / L->block[0];
     long long gy = (L->n[1] + L->block[1] - 1) / L->block[1];
     long long gz = (nfold + L->block[2] - 1) / L->block[2];
-    if (nred > 0) {  // reduction kernels stride over y/z (see the generated kernel)
-      long long cy = std::max(1LL, target / std::max(1LL, gx));
-      if (gy > cy) gy = cy;
-      long long cz = std::max(1LL, target / std::max(1LL, gx * gy));
-      if (gz > cz) gz = cz;
-    }
     if (nred == 0 && (gy > 65535 || gz > 65535))
       throw OPSException(OPS_NOT_IMPLEMENTED,
                          "Error: ops_par_loop range too large along y or z for one launch");
@@ -2495,22 +2493,59 @@ OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int d
     L->grid[1] = (int)gy;
     L->grid[2] = (int)gz;
   }
-  long long nblk = (long long)L->grid[0] * L->grid[1] * L->grid[2];
-  size_t need = red_bytes * (size_t)nblk + 256 * (size_t)nred;
-  if (need > r.partials_cap) {
-    if (r.partials) {
-      ob2_dev_sync();
-      ob2_dev_free(r.partials);
-    }
-    size_t cap = std::max(need, (size_t)1 << 20);
-    check(ob2_dev_malloc(&r.partials, cap), "reduction scratch");
-    r.partials_cap = cap;
-  }
   L->partials = r.partials;
   L->partials_bytes = r.partials_cap;
   L->counter = r.counter;
   L->ev_start = nullptr;  // launches are timed in ob2_launch / run_item
   return 1;
+}
+
+OPS_API unsigned ob2_red_grid(ob2_loop *L, int max_rows, int resident, unsigned tiles[3],
+                              int *rows) {
+  Runtime &r = rt();
+  long long nz = L->n[2];
+  for (int i = 0; i < 2; i++) nz *= std::max(0, L->hi4[i] - L->lo4[i]);
+  const long long ext[3] = {L->n[0], L->n[1], nz};
+  const long long wave = (long long)r.sms * resident * r.red_waves;
+  long long total;
+  // several rows per thread only where the tiles still fill the GPU (a CG's
+  // 200 x 177 update: 4.7 us with 1 row, 6.9 us with 4)
+  for (*rows = max_rows;; *rows = 1) {
+    const long long per[3] = {L->block[0], (long long)L->block[1] * *rows, L->block[2]};
+    total = 1;
+    for (int i = 0; i < 3; i++) {
+      tiles[i] = (unsigned)((ext[i] + per[i] - 1) / per[i]);
+      total *= tiles[i];
+    }
+    if (*rows == 1 || total >= wave) break;
+  }
+  // the trips spread evenly: with t tiles and w CTAs some CTA takes
+  // ceil(t / w) tiles, and the grid is the fewest CTAs that need no more
+  const long long trips = (total + wave - 1) / wave;
+  const long long grid = (total + trips - 1) / trips;
+  size_t bytes = 0;  // per CTA, one partial of each reduction argument
+  int nred = 0;
+  for (int i = 0; i < L->nargs; i++)
+    if (L->red[i].acc) {
+      bytes += (size_t)((ops_reduction)L->args[i].data)->size;
+      nred++;
+    }
+  // each argument's region is rounded up to 256 bytes by the stub
+  const size_t need = bytes * (size_t)grid + 256 * (size_t)nred;
+  if (need > r.partials_cap) {
+    if (r.partials) {
+      ob2_dev_sync();
+      ob2_dev_free(r.partials);
+      r.partials = nullptr;
+      r.partials_cap = 0;
+    }
+    const size_t cap = std::max(need, (size_t)1 << 20);
+    check(ob2_dev_malloc(&r.partials, cap), "reduction scratch");
+    r.partials_cap = cap;
+  }
+  L->partials = r.partials;
+  L->partials_bytes = r.partials_cap;
+  return (unsigned)grid;
 }
 
 OPS_API int ob2_args_alias(const ops_arg *args, int nargs) {

@@ -324,8 +324,8 @@ class Translator:
         # outweigh the few small register spills it causes)
         self.py_forced = "OPS_B200_PY" in os.environ
         self.py = max(1, int(os.environ.get("OPS_B200_PY", "1")))
-        # strided rows per trip of a reduction kernel's row loop (at least)
-        self.rpy = max(1, int(os.environ.get("OPS_B200_RPY", "1")))
+        # rows per thread and tile of a reduction kernel (0: by red_rows)
+        self.rpy = max(0, int(os.environ.get("OPS_B200_RPY", "0")))
         self.light_max = int(os.environ.get("OPS_B200_LIGHT", "4"))
         # OPS_B200_CHECK=1: OPS_ACCn accesses are checked against their dat's
         # allocation; an access outside it prints its kernel, argument, point
@@ -773,6 +773,20 @@ class Translator:
         widest = max([self.ELEM_BYTES.get(p.base_type, 8) for i, a, p in dats] or [8])
         return base * max(1, 8 // widest)
 
+    def red_rows(self, dats) -> int:
+        """Most consecutive rows per thread and tile of a reduction kernel:
+        4 when its dats read at most 24 bytes per point, so that a thread has
+        several rows' loads in flight, else 1 (the loads of one row are
+        enough, and more rows cost the registers that hold warps).  Measured
+        on one B200 at 4096^2, 1 / 2 / 4 / 8 rows: residual of a 5-point
+        stencil 80 / 63 / 59 / 60 us FP64 (16 B per point) and 79 / 60 / 46 /
+        42 us FP32, w = A p of a CG in FP32 (12 B) 98 / 94 / 71 / 77 us; the
+        FP64 residual with four dats (32 B) 138 / 150 / 166 / 167 us."""
+        if self.rpy:
+            return self.rpy
+        rd = sum(self.ELEM_BYTES.get(p.base_type, 8) for i, a, p in dats if a.acc != "OPS_WRITE")
+        return 4 if rd <= 24 else 1
+
     def align_dat(self, loop: Loop, kd, dats, reds, py):
         """3D loops without reductions and with one row per thread: the first
         written one-component dat of 4- or 8-byte elements, on whose rows the
@@ -949,6 +963,8 @@ class Translator:
             elif a.kind == "reduce":
                 w("  %s *r%d; %s *part%d; int first%d;" % (p.base_type, i, p.base_type, i, i))
                 reds.append((i, a, p))
+        if reds:  # tiles along x, y and z; rows per thread of a tile
+            w("  unsigned tx, ty, tz; int rows;")
         w("};")
         # Point function, in two variants: with __restrict__ dat pointers
         # (the common case: no dat is both written and passed twice, so the
@@ -1039,14 +1055,13 @@ class Translator:
         if reds:
             w("__global__ void __launch_bounds__(%s) %s(const __grid_constant__ %s p) {" %
               (lb, K, P))
-            w("  const unsigned bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;")
         else:
             # the body takes its CTA coordinates as arguments, so that one
             # launch can also run several instances of this loop (blocks of a
             # multi-block program) side by side: kernel <K>M below
             w("static __device__ __forceinline__ void %s(const %s &p, unsigned bx, unsigned by,"
               " unsigned bz) {" % (BF, P))
-        if aw is None:
+        if aw is None and not reds:
             w("  const int x = p.lo0 + (int)(bx * blockDim.x + threadIdx.x);")
         for i, a, p in reds:
             w("  %s red%d[%s];" % (p.base_type, i, a.dim))
@@ -1055,44 +1070,44 @@ class Translator:
         args_call = "".join(", p.b%d" % i for i, a, p in dats) + \
             "".join(", red%d" % i for i, a, p in reds)
         if reds:
-            py = max(py, self.rpy)
-            # reductions: grid of about one wave of resident CTAs, threads
-            # stride over y and z, so that few per-CTA partials are combined;
-            # PY strided rows per trip, so that their loads are in flight
-            # together
-            w("  if (x < p.hi0) {")
-            w("    const int ys = (int)(gridDim.y * blockDim.y) * %d;" % py)
+            py = self.red_rows(dats)
+            # reductions: one wave of resident CTAs (ob2_red_grid) walks the
+            # tiles of blockDim.x x (blockDim.y * PY) x blockDim.z points, so
+            # that few per-CTA partials are combined and no CTA waits for a
+            # second wave; PY consecutive rows per thread and tile keep that
+            # many rows' loads in flight
+            w("  const unsigned long long nt = (unsigned long long)p.tx * p.ty * p.tz;")
+            w("  for (unsigned long long t = blockIdx.x; t < nt; t += gridDim.x) {")
+            w("    unsigned bx, by, bz;")
+            w("    ob2::tile_of(t, nt, p.tx, p.ty, bx, by, bz);")
+            w("    const int x = p.lo0 + (int)(bx * blockDim.x + threadIdx.x);")
+            w("    const int yb = p.lo1 + (int)(by * blockDim.y + threadIdx.y) * p.rows;")
             if hd:  # the 3rd to 5th axes as one folded index
                 w("    const int nz = p.hi2 - p.lo2, nu = p.hi3 - p.lo3, nzu = nz * (p.hi4 - p.lo4) * nu;")
-                w("    for (int zz = (int)(bz * blockDim.z + threadIdx.z); zz < nzu;"
-                  " zz += (int)(gridDim.z * blockDim.z)) {")
-                w("      const int z = p.lo2 + zz % nz, u = p.lo3 + (zz / nz) % nu,"
+                w("    const int zz = (int)(bz * blockDim.z + threadIdx.z);")
+                w("    const int z = p.lo2 + zz % nz, u = p.lo3 + (zz / nz) % nu,"
                   " v = p.lo4 + zz / (nz * nu);")
+                w("    if (x < p.hi0 && zz < nzu) {")
             else:
-                w("    for (int z = p.lo2 + (int)(bz * blockDim.z + threadIdx.z); z < p.hi2;"
-                  " z += (int)(gridDim.z * blockDim.z))")
-            w("      for (int yb = p.lo1 + (int)(by * blockDim.y + threadIdx.y) * %d;"
-              " yb < p.hi1; yb += ys) {" % py)
-            # PY consecutive rows per trip; all in range: no branch between
-            # the calls, so the loads of every row can be issued before the
-            # stores of the first, and rows shared by the stencils are loaded
-            # once
+                w("    const int z = p.lo2 + (int)(bz * blockDim.z + threadIdx.z);")
+                w("    if (x < p.hi0 && z < p.hi2) {")
+            # all PY rows in range: no branch between the calls, so the loads
+            # of every row can be issued before the stores of the first, and
+            # rows shared by the stencils are loaded once
             zc = "z, u, v" if hd else "z"
-            w("        if (yb + %d < p.hi1) {" % (py - 1))
+            w("      if (p.rows == %d && yb + %d < p.hi1) {" % (py, py - 1))
             w("#pragma unroll")
-            w("          for (int j = 0; j < %d; j++) {" % py)
-            w("            if (RESTRICT) %s_R<IDX32>(p, x, yb + j, %s%s);" % (I, zc, args_call))
-            w("            else %s_A<IDX32>(p, x, yb + j, %s%s);" % (I, zc, args_call))
-            w("          }")
-            w("        } else {")
-            w("          for (int y = yb; y < p.hi1; y++) {")
-            w("            if (RESTRICT) %s_R<IDX32>(p, x, y, %s%s);" % (I, zc, args_call))
-            w("            else %s_A<IDX32>(p, x, y, %s%s);" % (I, zc, args_call))
-            w("          }")
+            w("        for (int j = 0; j < %d; j++) {" % py)
+            w("          if (RESTRICT) %s_R<IDX32>(p, x, yb + j, %s%s);" % (I, zc, args_call))
+            w("          else %s_A<IDX32>(p, x, yb + j, %s%s);" % (I, zc, args_call))
+            w("        }")
+            w("      } else {")
+            w("        for (int y = yb; y < min(yb + p.rows, p.hi1); y++) {")
+            w("          if (RESTRICT) %s_R<IDX32>(p, x, y, %s%s);" % (I, zc, args_call))
+            w("          else %s_A<IDX32>(p, x, y, %s%s);" % (I, zc, args_call))
             w("        }")
             w("      }")
-            if hd:
-                w("    }")
+            w("    }")
             w("  }")
         else:
             # PY points per thread along y (consecutive rows), x / z one each
@@ -1268,10 +1283,15 @@ class Translator:
               (128 // self.ELEM_BYTES[kd.params[aw].base_type] - 1))
         if not reds and py > 1:
             w("  grd.y = (L.n[1] + blk.y * %d - 1) / (blk.y * %d);" % (py, py))
-        elif reds and py > 1:
-            w("  grd.y = std::max(1u, std::min(grd.y, (unsigned)((L.n[1] + blk.y * %d - 1) /"
-              " (blk.y * %d))));" % (py, py))
         if reds:
+            w("  const bool al = ob2_args_alias(args, %d) != 0;" % na)
+            w("  const void *kern = al ? (L.idx32 ? (const void *)%s<false, true> : (const void *)%s"
+              "<false, false>) : (L.idx32 ? (const void *)%s<true, true> : (const void *)%s<true,"
+              " false>);" % (K, K, K, K))
+            w("  unsigned tiles[3];")
+            w("  grd = dim3(ob2_red_grid(&L, %d, ob2::resident_ctas(kern, (int)(blk.x * blk.y *"
+              " blk.z)), tiles, &p.rows), 1, 1);" % py)
+            w("  p.tx = tiles[0]; p.ty = tiles[1]; p.tz = tiles[2];")
             w("  size_t nblk = (size_t)grd.x * grd.y * grd.z;")
             w("  char *scratch = (char *)L.partials;")
         for i, (a, p) in enumerate(zip(loop.args, kd.params)):
@@ -1306,7 +1326,8 @@ class Translator:
                 w("  p.part%d = (%s *)scratch;"
                   " scratch += ((nblk * (%s) * sizeof(%s) + 255) / 256) * 256;" %
                   (i, p.base_type, a.dim, p.base_type))
-        w("  const bool al = ob2_args_alias(args, %d) != 0;" % na)
+        if not reds:
+            w("  const bool al = ob2_args_alias(args, %d) != 0;" % na)
         w("  const ob2_launcher fn = al ? (L.idx32 ? %s_f_t : %s_f_f)"
           " : (L.idx32 ? %s_t_t : %s_t_f);" % (LN, LN, LN, LN))
         w("  const unsigned g3[3] = {grd.x, grd.y, grd.z}, b3[3] = {blk.x, blk.y, blk.z};")
