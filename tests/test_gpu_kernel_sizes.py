@@ -61,3 +61,77 @@ def test_trid_too_long_is_refused():
         strides = (C.c_longlong * 3)(1, dims[0], dims[0] * dims[1])
         assert L.ob2_trid_batch(8, 3, dim, cabi.ivec(dims), strides, None, None, None, None,
                                 None) != 0
+
+
+BOXES = [(1, 1, 1), (1, 7, 5), (2, 3, 4), (5, 1, 8), (31, 4, 2), (33, 6, 3), (40, 9, 8)]
+
+
+@pytest.mark.parametrize("soa", [0, 1])
+@pytest.mark.parametrize("typ", ["double", "float", "int", "half", "complexd"])
+@pytest.mark.parametrize("dim", [1, 2, 3, 5])
+def test_slab_fetch_and_set(soa, typ, dim):
+    """Boxes of a 3D dat out and back through host buffers: rows from one
+    element to the whole width, every component count and element size (2 to
+    16 bytes), AoS and SoA; bytes equal to the numpy slice, nothing outside
+    the box written."""
+    import ctypes as C
+
+    import numpy as np
+
+    from tests import cabi
+    L = cabi.lib()
+    ts = {"double": 8, "float": 4, "int": 4, "half": 2, "complexd": 16}[typ]
+    vp, ip = C.c_void_p, C.POINTER(C.c_int)
+    for f in (L.ops_dat_fetch_data_slab_memspace, L.ops_dat_set_data_slab_memspace):
+        f.argtypes = [vp, C.c_int, vp, ip, C.c_int]
+    n = [40, 9, 8]
+    blk = L.ops_decl_block(3, b"box")
+    L.ops_set_soa(soa)
+    try:
+        h = L.ops_decl_dat_char(blk, dim, cabi.ivec(n), cabi.ivec([0] * 3), cabi.ivec([-1] * 3),
+                                cabi.ivec([1] * 3), cabi.ivec([1] * 3), None, ts, typ.encode(),
+                                b"box")
+        rng = np.random.default_rng(dim * 100 + ts)
+        model = rng.integers(0, 256, (n[2], n[1], n[0], dim * ts), dtype=np.uint8)
+        whole = cabi.ivec([0, n[0], 0, n[1], 0, n[2]])
+        L.ops_dat_set_data_slab_memspace(h, 0, model.ctypes.data, whole, 1)
+        for k, b in enumerate(BOXES):
+            lo = [int(rng.integers(0, n[i] - b[i] + 1)) for i in range(3)]
+            r = cabi.ivec([v for i in range(3) for v in (lo[i], lo[i] + b[i])])
+            sl = tuple(slice(lo[i], lo[i] + b[i]) for i in (2, 1, 0))
+            got = np.empty((b[2], b[1], b[0], dim * ts), np.uint8)
+            L.ops_dat_fetch_data_slab_memspace(h, 0, got.ctypes.data, r, 1)
+            assert np.array_equal(got, model[sl]), (b, lo)
+            new = rng.integers(0, 256, got.shape, dtype=np.uint8)
+            L.ops_dat_set_data_slab_memspace(h, 0, new.ctypes.data, r, 1)
+            model[sl] = new
+            back = np.empty_like(model)
+            L.ops_dat_fetch_data_slab_memspace(h, 0, back.ctypes.data, whole, 1)
+            assert np.array_equal(back, model), (b, lo)
+    finally:
+        L.ops_set_soa(0)
+
+
+def test_slab_of_long_rows():
+    """Rows of more than one piece (1024 units of 8 bytes), 1D and 2D."""
+    import ctypes as C
+
+    import numpy as np
+
+    from tests import cabi
+    L = cabi.lib()
+    vp, ip = C.c_void_p, C.POINTER(C.c_int)
+    for f in (L.ops_dat_fetch_data_slab_memspace, L.ops_dat_set_data_slab_memspace):
+        f.argtypes = [vp, C.c_int, vp, ip, C.c_int]
+    for n, lo, hi in (([5003], [2], [5001]), ([1025, 3], [0, 1], [1025, 3]),
+                      ([4097, 2], [1, 0], [4096, 2])):
+        nd = len(n)
+        blk = L.ops_decl_block(nd, b"rows")
+        d = cabi.Dat(blk, nd, n, [-1] * nd, [1] * nd, "double", "rows")
+        a = np.random.default_rng(3).random(n[::-1])
+        d.set_interior(a)
+        sl = tuple(slice(lo[i], hi[i]) for i in reversed(range(nd)))
+        got = np.empty(a[sl].shape)
+        r = cabi.ivec([v for i in range(nd) for v in (lo[i], hi[i])])
+        L.ops_dat_fetch_data_slab_memspace(d.h, 0, got.ctypes.data, r, 1)
+        assert np.array_equal(got, a[sl])
