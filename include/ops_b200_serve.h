@@ -19,14 +19,13 @@
  *                   added to u), u0 ~ U(-1,1) from the seed.
  *
  * Every admitted request keeps its arrays resident in HBM until released.
- * All active requests advance together: one engine iteration is one launch
- * of each batched kernel over a device-side work list that spans every
- * active request (ragged sizes share the launch), and the CG scalars live on
- * the device, so an iteration needs no host round trip.  `ob2s_run` replays
- * one CUDA graph of K iterations; the graph reads the work list from device
- * memory, so it stays valid when requests join or leave (continuous
- * batching: new requests join at the next ob2s_run, finished ones stop
- * consuming work immediately).
+ * All active requests advance together over a device-side work list that
+ * spans every active request (ragged sizes share the launches), and the CG
+ * scalars live on the device, so an iteration needs no host round trip.
+ * `ob2s_run` runs K iterations: one cooperative launch for all CG iterations
+ * (a CTA per SM, grid barriers between the passes), three launches per ADI
+ * step.  New requests join at the next ob2s_run, finished ones stop
+ * consuming work immediately (continuous batching).
  *
  * Precision modes (conjugate gradients, FP64 iterate x):
  *   OB2S_FP64   CG in FP64 (the plain form);
@@ -75,7 +74,7 @@ typedef struct ob2s_result {
 } ob2s_result;
 
 /* tile_y: rows of a Poisson tile (8, 16 or 32 = 1, 2 or 4 rows per thread of
- * a 32 x 8 CTA; 0 = 32). */
+ * a 32 x 8 group; 0 = 32). */
 OB2_API int ob2s_create(ob2s_engine **e, int mode, double tol, double inner_tol, int max_inner,
                         int tile_y);
 OB2_API void ob2s_destroy(ob2s_engine *e);
@@ -89,8 +88,7 @@ OB2_API size_t ob2s_request_bytes(int mode, int kind, int n);
  * set at the next ob2s_run.  steps: ADI or heat time steps (ignored for
  * Poisson). */
 OB2_API int ob2s_submit(ob2s_engine *e, int kind, int n, int seed, int steps, int *id);
-/* Runs `iters` engine iterations (a graph of that many is captured once per
- * value and replayed) and waits for them; *n_done: requests finished since
+/* Runs `iters` engine iterations and waits for them; *n_done: requests finished since
  * the last call, their ids in ids[0..cap). */
 OB2_API int ob2s_run(ob2s_engine *e, int iters, int *ids, int cap, int *n_done);
 OB2_API int ob2s_active(ob2s_engine *e);
@@ -99,7 +97,7 @@ OB2_API int ob2s_result_of(ob2s_engine *e, int id, ob2s_result *res);
 OB2_API int ob2s_fetch(ob2s_engine *e, int id, double *host, size_t count);
 /* frees the request's device memory and its slot */
 OB2_API int ob2s_release(ob2s_engine *e, int id);
-/* kernel launches issued by the engine (graph replays count their kernels) */
+/* kernel launches issued by the engine */
 OB2_API long long ob2s_launches(ob2s_engine *e);
 
 #endif /* OPS_B200_SERVE_H */

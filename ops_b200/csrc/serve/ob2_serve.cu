@@ -2,20 +2,19 @@
 //
 // Device state: an array of request slots (struct Req, FP64 CG scalars
 // included) and a work list (struct Work) naming the active requests with
-// prefix sums of their work units.  Every batched kernel is persistent: a
-// grid of a few CTAs per SM walks the global unit index over all active
-// requests, finds the request by binary search in the prefix table, and works
-// on that request's tile.  One engine iteration:
-//   pois_pw       p' = r + beta p, w = A p', per-tile (p', w)
-//   scalars_a     alpha per Poisson request
-//   pois_xr       x += alpha p' (FP64), r -= alpha w, per-tile (r, r); or
-//                 the FP64 residual b - A x
-//   adi_pre       right-hand side of the ADI step (adi/preproc_kernel.h)
-//   adi_x/y/z     constant-coefficient Thomas solves (z adds into u)
-//   scalars_b     per request: fixed-order sum of its tile partials, beta,
-//                 residual replacement and convergence; ADI step count
-// All kernels read the work list from device memory, so one captured graph
-// of K iterations serves every batch composition.
+// prefix sums of their work units.  One call of ob2s_run is
+//   pois_iterate  one cooperative launch that runs all the iterations of the
+//                 Poisson and heat requests: every CTA owns a run of tiles of
+//                 the work list; per iteration p' = r + beta p, w = A p' and
+//                 per-tile (p', w), a grid barrier, x += alpha p', r -= alpha
+//                 w and per-tile (r, r) (or the FP64 residual b - A x), a
+//                 grid barrier.  Each CTA forms alpha, beta and the state
+//                 changes of its own requests from all their tile partials,
+//                 in a fixed order, so that all CTAs of a request agree;
+//   adi_x/y/z     three launches per ADI step: right-hand side and x solve,
+//                 y solve, z solve added into u (chunks in registers, PCR
+//                 among the lanes of a line), then adi_count once.
+// All kernels read the work list from device memory.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -25,23 +24,26 @@
 #include <algorithm>
 #include <vector>
 
+#include "../device/ob2_trid.cuh"
 #include "ops_b200_serve.h"
 
 namespace {
+
+using namespace ob2t;
 
 constexpr int TX = 32;       // CTA x extent (one warp per row of a tile)
 constexpr int TXC = 2 * TX;  // columns per tile: two adjacent columns per thread
 constexpr int C0 = 2;        // storage column of interior column 0 (even: 2-column
                              // accesses are 8- or 16-byte aligned)
 constexpr int MAXA = OB2S_MAX_ACTIVE;
-constexpr int ADI_MAX_N = 192;  // x-solve tile: 32 lines x n points in shared memory
-constexpr int ADI_XL = 32;      // lines per x-solve unit
+constexpr int ADI_MAX_N = 192;  // 32 lanes x 6 points
+constexpr int ADI_CL = 6;       // points per chunk of a line
 // (OB2S_HEAT2D is declared in ops_b200_serve.h)
-constexpr int ADI_YZ = 4;       // planes per y/z-solve unit (CTA 32 x 4 lines)
 constexpr double kHeatRho = 1.0;  // heat requests: dt / h^2 of the implicit step
 
 struct Req {
   int kind, n, pitch, tiles_x, tiles;
+  int ry;   // 2D: rows per thread of a tile (1, 2 or 4); ADI: lanes per line (8, 16 or 32)
   int phase, done, outer, inner_it, iters;
   int max_inner, max_outer, steps, step;
   int par;  // p buffer parity
@@ -51,8 +53,8 @@ struct Req {
   double diag, off;  // heat operator: diag x - off (sum of the 4 neighbours)
   double *x, *b, *part;
   void *r, *w, *p0, *p1;
-  double *u, *du, *cp, *mm;
-  double a_coef, lambda;
+  double *u, *du;
+  double lambda;
 };
 
 struct Work {
@@ -60,9 +62,7 @@ struct Work {
   int pois_slot[MAXA];
   int adi_slot[MAXA];
   long long pois_pref[MAXA + 1];
-  long long pre_pref[MAXA + 1];
-  long long x_pref[MAXA + 1];
-  long long yz_pref[MAXA + 1];
+  long long adi_pref[MAXA + 1];
 };
 
 __device__ __forceinline__ int find_req(const long long *pref, int n, long long u) {
@@ -93,11 +93,12 @@ __device__ __forceinline__ double hash_uniform(int seed, int i, int j, int k) {
 // storage rows 0 .. n+1, row pitch P even and at least n + 3, interior
 // column i at storage column i + C0 (column -1, the left halo, at C0 - 1;
 // column n, the right halo, at n + C0); every unused element is zero.
-// CTA 32 x 8 threads; each thread handles two adjacent columns (one 8- or
-// 16-byte access per array and row) and RY consecutive rows, so a tile is
-// 64 x (8 RY) points.  Loads of out-of-range rows are clamped to the last
-// interior row (always valid memory) and only the stores are guarded, so the
-// loads of all RY rows are issued before any store.
+// A tile is worked on by a group of 32 x 8 threads; each thread handles two
+// adjacent columns (one 8- or 16-byte access per array and row) and RY
+// consecutive rows, so a tile is 64 x (8 RY) points.  Loads of out-of-range
+// rows are clamped to the last interior row (always valid memory) and only
+// the stores are guarded, so the loads of all RY rows are issued before any
+// store.
 //
 // Poisson and heat requests: conjugate gradients (the standard
 // two-reduction form) with the iterate x in FP64, the vectors r, w, p in TI
@@ -114,14 +115,14 @@ __device__ __forceinline__ double hash_uniform(int seed, int i, int j, int k) {
 // Phases:
 //   0  start (and restart after a breakdown; for heat requests also the start
 //      of each time step, which first sets b = x): r = b - A x in FP64
-//   2  CG iteration: p' = r + beta p, w = A p', (p', w)   [pois_pw]
-//                    alpha = gamma / (p', w)               [scalars_a]
-//                    x += alpha p', r -= alpha w, (r, r)   [pois_xr]
-//                    beta, gamma; replacement test         [scalars_b]
+//   2  CG iteration: p' = r + beta p, w = A p', (p', w)   [pw_tile]
+//                    alpha = gamma / (p', w)               [form_alpha]
+//                    x += alpha p', r -= alpha w, (r, r)   [xr_tile]
+//                    beta, gamma; replacement test         [advance]
 //   3  replacement: r = b - A x in FP64, convergence test on it; beta from
 //      the true (r, r), p kept
-// p is double-buffered (p[par] read, p[par ^ 1] written by pois_pw), since
-// pois_pw forms p' of the stencil neighbours itself: w = A p' needs p' at
+// p is double-buffered (p[par] read, p[par ^ 1] written by pw_tile), since
+// pw_tile forms p' of the stencil neighbours itself: w = A p' needs p' at
 // the neighbours, and recomputing r + beta p there avoids a separate pass.
 
 constexpr int CTA_Y = 8;
@@ -143,13 +144,41 @@ __device__ __forceinline__ void st2(T *p, T a, T b) {
   *(typename V2<T>::type *)p = v;
 }
 
-// resident CTAs per SM the Poisson kernels are compiled for (register cap):
-// 4 for FP32 vectors; 3 for FP64 ones, whose two columns of RY rows need
-// more than 64 registers without spilling
-#ifndef OB2S_MINB
-#define OB2S_MINB 4
-#endif
-#define POIS_BOUNDS __launch_bounds__(256, sizeof(TI) == 8 ? 3 : OB2S_MINB)
+// Groups of 256 threads per CTA, one CTA per SM: 4 for FP32 vectors (64
+// registers a thread), 3 for FP64 ones, whose two columns of RY rows need
+// more than 64
+constexpr int GT = TX * CTA_Y;  // threads of a group
+template <typename TI>
+__host__ __device__ constexpr int pois_groups() {
+  return sizeof(TI) == 8 ? 3 : 4;
+}
+
+// a group's own barrier (every group of the CTA takes its tiles at its pace)
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(GT) : "memory");
+}
+
+// fixed-order sum over a group of NV values per thread; result in thread 0
+template <int NV>
+__device__ __forceinline__ void group_sum(double (&v)[NV], double (*sh)[CTA_Y], int g) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < NV; c++) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+  const int t = threadIdx.x % GT;
+  if ((t & 31) == 0)
+#pragma unroll
+    for (int c = 0; c < NV; c++) sh[c][t >> 5] = v[c];
+  group_sync(g);
+  if (t == 0)
+#pragma unroll
+    for (int c = 0; c < NV; c++) {
+      double a = 0.0;
+      for (int k = 0; k < CTA_Y; k++) a += sh[c][k];
+      v[c] = a;
+    }
+  group_sync(g);
+}
 
 // fixed-order CTA sum of NV values per thread; result in thread 0
 template <int NV>
@@ -174,210 +203,188 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double (*sh)[32]) {
   __syncthreads();
 }
 
-// p' = r + beta p and w = A p' over the tile, (p', w) per tile (phase 2)
+// What the CTAs that work on a request keep of it in shared memory: its
+// arrays and operator (constant), and its CG state, which each of them
+// advances by itself from the same partial sums.
+struct Pois {
+  int kind, n, pitch, tiles_x, tiles, ry;
+  int phase, done, outer, iters, step, par, newstep;
+  int max_inner, max_outer, steps;
+  double tol, inner_tol, diag, off;
+  double alpha, beta, gamma, gamma_in0, rr0, rel;
+  double *x, *b, *part;
+  void *r, *w, *p0, *p1;
+};
+
+// p' = r + beta p and w = A p' over tile t, (p', w) of the tile (phase 2)
 template <typename TI, int RY>
-__global__ void POIS_BOUNDS pois_pw(const Work *__restrict__ W, Req *R) {
-  __shared__ double sh[1][32];
-  const long long total = W->pois_pref[W->npois];
-  for (long long un = blockIdx.x; un < total; un += gridDim.x) {
-    const int k = find_req(W->pois_pref, W->npois, un);
-    const Req &q = R[W->pois_slot[k]];
-    if (q.done || q.phase != 2) continue;  // uniform over the CTA
-    const int t = (int)(un - W->pois_pref[k]);
-    const int n = q.n, P = q.pitch;
-    const int i = (t % q.tiles_x) * TXC + 2 * threadIdx.x;  // columns i, i + 1
-    const int j0 = (t / q.tiles_x) * (CTA_Y * RY) + threadIdx.y * RY;
-    double v[1] = {0.0};
-    if (j0 < n) {  // uniform over the warp (one threadIdx.y per warp)
-      const TI *rr = (const TI *)q.r;
-      const TI *pin = (const TI *)(q.par ? q.p1 : q.p0);
-      TI *pout = (TI *)(q.par ? q.p0 : q.p1);
-      TI *ww = (TI *)q.w;
-      const TI beta = (TI)q.beta;
-      const bool in0 = i < n, in1 = i + 1 < n;
-      const int ic = in0 ? i : ((n - 1) & ~1);  // lanes past the edge load valid memory
-      const int lane = threadIdx.x;
-      // p' = r + beta p on rows j0-1 .. j0+RY of columns i, i+1 (storage rows
-      // clamped into the array; the halo rows and columns of r and p hold
-      // zeros); a column past the right edge stands for the zero halo
-      TI p0[RY + 2], p1[RY + 2];
-      int o[RY + 2];  // (n + 2) P < 2^31 for n <= 32768
+__device__ __forceinline__ void pw_tile(const Pois &q, int t, int g, double (*sh)[CTA_Y]) {
+  const int lane = threadIdx.x % TX, ty = threadIdx.x % GT / TX;
+  const int n = q.n, P = q.pitch;
+  const int i = (t % q.tiles_x) * TXC + 2 * lane;  // columns i, i + 1
+  const int j0 = (t / q.tiles_x) * (CTA_Y * RY) + ty * RY;
+  double v[1] = {0.0};
+  if (j0 < n) {  // uniform over the warp (one row of a tile per warp)
+    const TI *rr = (const TI *)q.r;
+    const TI *pin = (const TI *)(q.par ? q.p1 : q.p0);
+    TI *pout = (TI *)(q.par ? q.p0 : q.p1);
+    TI *ww = (TI *)q.w;
+    const TI beta = (TI)q.beta;
+    const bool in0 = i < n, in1 = i + 1 < n;
+    const int ic = in0 ? i : ((n - 1) & ~1);  // lanes past the edge load valid memory
+    // p' = r + beta p on rows j0-1 .. j0+RY of columns i, i+1 (storage rows
+    // clamped into the array; the halo rows and columns of r and p hold
+    // zeros); a column past the right edge stands for the zero halo
+    TI p0[RY + 2], p1[RY + 2];
+    int o[RY + 2];  // (n + 2) P < 2^31 for n <= 32768
 #pragma unroll
-      for (int m = 0; m < RY + 2; m++) {
-        o[m] = (min(j0 + m - 1, n) + 1) * P + ic + C0;
-        const auto rv = ld2(rr + o[m]);
-        const auto pv = ld2(pin + o[m]);
-        p0[m] = in0 ? rv.x + beta * pv.x : (TI)0;
-        p1[m] = in1 ? rv.y + beta * pv.y : (TI)0;
-      }
-#pragma unroll
-      for (int m = 0; m < RY; m++) {
-        // column i - 1 is the left lane's second column, column i + 2 the
-        // right lane's first; the warp's edge lanes form theirs from memory
-        // (the same arithmetic, same bits)
-        TI pw = __shfl_up_sync(0xffffffffu, p1[m + 1], 1);
-        TI pe = __shfl_down_sync(0xffffffffu, p0[m + 1], 1);
-        if (lane == 0) pw = rr[o[m + 1] - 1] + beta * pin[o[m + 1] - 1];
-        if (lane == TX - 1 && in1) pe = rr[o[m + 1] + 2] + beta * pin[o[m + 1] + 2];
-        if (!in0 || j0 + m >= n) continue;
-        const TI c0 = p0[m + 1], c1 = p1[m + 1];
-        TI a0, a1;
-        if (q.kind == OB2S_HEAT2D) {
-          a0 = (TI)q.diag * c0 - (TI)q.off * (pw + c1 + p0[m] + p0[m + 2]);
-          a1 = in1 ? (TI)q.diag * c1 - (TI)q.off * (c0 + pe + p1[m] + p1[m + 2]) : (TI)0;
-        } else {
-          a0 = (TI)4 * c0 - pw - c1 - p0[m] - p0[m + 2];
-          a1 = in1 ? (TI)4 * c1 - c0 - pe - p1[m] - p1[m + 2] : (TI)0;
-        }
-        // column n (the right halo) gets zeros when i + 1 == n
-        st2(pout + o[m + 1], c0, c1);
-        st2(ww + o[m + 1], a0, a1);
-        v[0] += (double)c0 * (double)a0 + (double)c1 * (double)a1;
-      }
+    for (int m = 0; m < RY + 2; m++) {
+      o[m] = (min(j0 + m - 1, n) + 1) * P + ic + C0;
+      const auto rv = ld2(rr + o[m]);
+      const auto pv = ld2(pin + o[m]);
+      p0[m] = in0 ? rv.x + beta * pv.x : (TI)0;
+      p1[m] = in1 ? rv.y + beta * pv.y : (TI)0;
     }
-    block_sum<1>(v, sh);
-    if (threadIdx.x == 0 && threadIdx.y == 0) q.part[NPART * t] = v[0];
+#pragma unroll
+    for (int m = 0; m < RY; m++) {
+      // column i - 1 is the left lane's second column, column i + 2 the
+      // right lane's first; the warp's edge lanes form theirs from memory
+      // (the same arithmetic, same bits)
+      TI pw = __shfl_up_sync(0xffffffffu, p1[m + 1], 1);
+      TI pe = __shfl_down_sync(0xffffffffu, p0[m + 1], 1);
+      if (lane == 0) pw = rr[o[m + 1] - 1] + beta * pin[o[m + 1] - 1];
+      if (lane == TX - 1 && in1) pe = rr[o[m + 1] + 2] + beta * pin[o[m + 1] + 2];
+      if (!in0 || j0 + m >= n) continue;
+      const TI c0 = p0[m + 1], c1 = p1[m + 1];
+      TI a0, a1;
+      if (q.kind == OB2S_HEAT2D) {
+        a0 = (TI)q.diag * c0 - (TI)q.off * (pw + c1 + p0[m] + p0[m + 2]);
+        a1 = in1 ? (TI)q.diag * c1 - (TI)q.off * (c0 + pe + p1[m] + p1[m + 2]) : (TI)0;
+      } else {
+        a0 = (TI)4 * c0 - pw - c1 - p0[m] - p0[m + 2];
+        a1 = in1 ? (TI)4 * c1 - c0 - pe - p1[m] - p1[m + 2] : (TI)0;
+      }
+      // column n (the right halo) gets zeros when i + 1 == n
+      st2(pout + o[m + 1], c0, c1);
+      st2(ww + o[m + 1], a0, a1);
+      v[0] += (double)c0 * (double)a0 + (double)c1 * (double)a1;
+    }
   }
+  group_sum<1>(v, sh, g);
+  if (threadIdx.x % GT == 0) q.part[NPART * t] = v[0];
 }
 
 // phase 2: x += alpha p' (FP64), r -= alpha w, (r, r); phases 0, 3:
 // r = b - A x in FP64 and its (r, r).  Column n (the right halo) is written
 // only with zeros: there p', w and r are zero, so x keeps its zero.
 template <typename TI, int RY>
-__global__ void POIS_BOUNDS pois_xr(const Work *__restrict__ W, Req *R) {
-  __shared__ double sh[2][32];
-  const long long total = W->pois_pref[W->npois];
-  for (long long un = blockIdx.x; un < total; un += gridDim.x) {
-    const int k = find_req(W->pois_pref, W->npois, un);
-    const Req &q = R[W->pois_slot[k]];
-    if (q.done) continue;  // uniform over the CTA
-    const int ph = q.phase;
-    const int t = (int)(un - W->pois_pref[k]);
-    const int n = q.n, P = q.pitch;
-    const int i = (t % q.tiles_x) * TXC + 2 * threadIdx.x;  // columns i, i + 1
-    const int j0 = (t / q.tiles_x) * (CTA_Y * RY) + threadIdx.y * RY;
-    double v[2] = {0.0, 0.0};
-    if (i < n && j0 < n) {
-      const bool in1 = i + 1 < n;
-      int o[RY];  // (n + 2) P < 2^31 for n <= 32768
+__device__ __forceinline__ void xr_tile(const Pois &q, int t, int g, double (*sh)[CTA_Y]) {
+  const int lane = threadIdx.x % TX, ty = threadIdx.x % GT / TX;
+  const int ph = q.phase;
+  const int n = q.n, P = q.pitch;
+  const int i = (t % q.tiles_x) * TXC + 2 * lane;  // columns i, i + 1
+  const int j0 = (t / q.tiles_x) * (CTA_Y * RY) + ty * RY;
+  double v[2] = {0.0, 0.0};
+  if (i < n && j0 < n) {
+    const bool in1 = i + 1 < n;
+    int o[RY];  // (n + 2) P < 2^31 for n <= 32768
 #pragma unroll
-      for (int m = 0; m < RY; m++) o[m] = (min(j0 + m, n - 1) + 1) * P + i + C0;
-      TI *rr = (TI *)q.r;
-      double *x = q.x;
-      if (ph == 2) {
-        const TI *pn = (const TI *)(q.par ? q.p0 : q.p1);  // written by pois_pw
-        const TI *ww = (const TI *)q.w;
-        const double alpha64 = q.alpha;
-        const TI alpha = (TI)q.alpha;
-        double x0[RY], x1[RY];
-        TI r0[RY], r1[RY];
+    for (int m = 0; m < RY; m++) o[m] = (min(j0 + m, n - 1) + 1) * P + i + C0;
+    TI *rr = (TI *)q.r;
+    double *x = q.x;
+    if (ph == 2) {
+      const TI *pn = (const TI *)(q.par ? q.p0 : q.p1);  // written by pw_tile
+      const TI *ww = (const TI *)q.w;
+      const double alpha64 = q.alpha;
+      const TI alpha = (TI)q.alpha;
+      double x0[RY], x1[RY];
+      TI r0[RY], r1[RY];
 #pragma unroll
-        for (int m = 0; m < RY; m++) {
-          const auto pv = ld2(pn + o[m]);
-          const auto wv = ld2(ww + o[m]);
-          const auto rv = ld2(rr + o[m]);
-          const double2 xv = ld2(x + o[m]);
-          x0[m] = xv.x + alpha64 * (double)pv.x;
-          x1[m] = xv.y + alpha64 * (double)pv.y;
-          r0[m] = rv.x - alpha * wv.x;
-          r1[m] = rv.y - alpha * wv.y;
-        }
+      for (int m = 0; m < RY; m++) {
+        const auto pv = ld2(pn + o[m]);
+        const auto wv = ld2(ww + o[m]);
+        const auto rv = ld2(rr + o[m]);
+        const double2 xv = ld2(x + o[m]);
+        x0[m] = xv.x + alpha64 * (double)pv.x;
+        x1[m] = xv.y + alpha64 * (double)pv.y;
+        r0[m] = rv.x - alpha * wv.x;
+        r1[m] = rv.y - alpha * wv.y;
+      }
 #pragma unroll
-        for (int m = 0; m < RY; m++) {
-          if (j0 + m >= n) continue;
-          st2(x + o[m], x0[m], x1[m]);
-          st2(rr + o[m], r0[m], r1[m]);
-          v[0] += (double)r0[m] * (double)r0[m] + (double)r1[m] * (double)r1[m];
-        }
-      } else {
-        double *b = q.b;
-        double s0[RY], s1[RY];
+      for (int m = 0; m < RY; m++) {
+        if (j0 + m >= n) continue;
+        st2(x + o[m], x0[m], x1[m]);
+        st2(rr + o[m], r0[m], r1[m]);
+        v[0] += (double)r0[m] * (double)r0[m] + (double)r1[m] * (double)r1[m];
+      }
+    } else {
+      double *b = q.b;
+      double s0[RY], s1[RY];
 #pragma unroll
-        for (int m = 0; m < RY; m++) {
-          const int e = o[m];
-          const double2 c = ld2(x + e), up = ld2(x + e - P), dn = ld2(x + e + P);
-          const double xw = x[e - 1], xe = x[e + 2];
-          double2 bv = ld2(b + e);
-          if (q.kind == OB2S_HEAT2D) {
-            if (q.newstep) {  // a new time step: its right-hand side is the last solution
-              bv = c;
-              if (j0 + m < n) {
-                st2(b + e, bv.x, bv.y);
-                v[1] += bv.x * bv.x + bv.y * bv.y;  // ||b||^2: the step's residuals are relative to it
-              }
+      for (int m = 0; m < RY; m++) {
+        const int e = o[m];
+        const double2 c = ld2(x + e), up = ld2(x + e - P), dn = ld2(x + e + P);
+        const double xw = x[e - 1], xe = x[e + 2];
+        double2 bv = ld2(b + e);
+        if (q.kind == OB2S_HEAT2D) {
+          if (q.newstep) {  // a new time step: its right-hand side is the last solution
+            bv = c;
+            if (j0 + m < n) {
+              st2(b + e, bv.x, bv.y);
+              v[1] += bv.x * bv.x + bv.y * bv.y;  // ||b||^2: the step's residuals are relative to it
             }
-            s0[m] = bv.x - (q.diag * c.x - q.off * (xw + c.y + up.x + dn.x));
-            s1[m] = in1 ? bv.y - (q.diag * c.y - q.off * (c.x + xe + up.y + dn.y)) : 0.0;
-          } else {
-            s0[m] = bv.x - (4.0 * c.x - xw - c.y - up.x - dn.x);
-            s1[m] = in1 ? bv.y - (4.0 * c.y - c.x - xe - up.y - dn.y) : 0.0;
           }
-        }
-#pragma unroll
-        for (int m = 0; m < RY; m++) {
-          if (j0 + m >= n) continue;
-          st2(rr + o[m], (TI)s0[m], (TI)s1[m]);
-          v[0] += s0[m] * s0[m] + s1[m] * s1[m];
+          s0[m] = bv.x - (q.diag * c.x - q.off * (xw + c.y + up.x + dn.x));
+          s1[m] = in1 ? bv.y - (q.diag * c.y - q.off * (c.x + xe + up.y + dn.y)) : 0.0;
+        } else {
+          s0[m] = bv.x - (4.0 * c.x - xw - c.y - up.x - dn.x);
+          s1[m] = in1 ? bv.y - (4.0 * c.y - c.x - xe - up.y - dn.y) : 0.0;
         }
       }
+#pragma unroll
+      for (int m = 0; m < RY; m++) {
+        if (j0 + m >= n) continue;
+        st2(rr + o[m], (TI)s0[m], (TI)s1[m]);
+        v[0] += s0[m] * s0[m] + s1[m] * s1[m];
+      }
     }
-    block_sum<2>(v, sh);
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-      q.part[NPART * t + 1] = v[0];
-      // column 0 is free in phase 0 (pois_pw did not run): ||b||^2 of a new
-      // heat time step
-      if (ph == 0 && q.newstep) q.part[NPART * t] = v[1];
-    }
+  }
+  group_sum<2>(v, sh, g);
+  if (threadIdx.x % GT == 0) {
+    q.part[NPART * t + 1] = v[0];
+    // column 0 is free in phase 0 (pw_tile did not run): ||b||^2 of a new
+    // heat time step
+    if (ph == 0 && q.newstep) q.part[NPART * t] = v[1];
   }
 }
 
-// per-request fixed-order sum of one partial column
-__device__ __forceinline__ double request_sum(const Req &q, int col, double (*sh)[32]) {
+// a group's fixed-order sum of one partial column of a request (in thread 0)
+__device__ __forceinline__ double request_sum(const Pois &q, int col, double (*sh)[CTA_Y], int g) {
   double v[1] = {0.0};
-  for (int t = threadIdx.x; t < q.tiles; t += blockDim.x) v[0] += q.part[NPART * t + col];
-  block_sum<1>(v, sh);
+  for (int t = threadIdx.x % GT; t < q.tiles; t += GT) v[0] += q.part[NPART * t + col];
+  group_sum<1>(v, sh, g);
   return v[0];
 }
 
-// alpha = gamma / (p', w) for requests in phase 2
-__global__ void __launch_bounds__(256) scalars_a(const Work *__restrict__ W, Req *R) {
-  __shared__ double sh[1][32];
-  const int b = blockIdx.x;
-  if (b >= W->npois) return;
-  Req &q = R[W->pois_slot[b]];
-  if (q.done || q.phase != 2) return;
-  const double pw = request_sum(q, 0, sh);
-  if (threadIdx.x != 0) return;
-  if (!(pw > 0.0)) {  // breakdown: pois_xr computes the true residual and
-    q.phase = 0;       // scalars_b restarts from it with beta = 0
-    return;
-  }
-  q.alpha = q.gamma / pw;
+// alpha = gamma / (p', w) of a request in phase 2
+__device__ __forceinline__ void form_alpha(Pois &q, double (*sh)[CTA_Y], int g) {
+  if (q.done || q.phase != 2) return;  // uniform over the group
+  const double pw = request_sum(q, 0, sh, g);
+  if (threadIdx.x % GT != 0) return;
+  if (!(pw > 0.0))  // breakdown: xr_tile computes the true residual and
+    q.phase = 0;    // advance restarts from it with beta = 0
+  else
+    q.alpha = q.gamma / pw;
 }
 
-// (r, r) step of every Poisson request; CTAs [MAXA, MAXA + nadi) advance
-// the ADI requests' step counts
-__global__ void __launch_bounds__(256) scalars_b(const Work *__restrict__ W, Req *R) {
-  __shared__ double sh[1][32];
-  const int b = blockIdx.x;
-  if (b >= MAXA) {
-    const int k = b - MAXA;
-    if (k >= W->nadi || threadIdx.x != 0) return;
-    Req &q = R[W->adi_slot[k]];
-    if (q.done) return;
-    q.step++;
-    q.iters = q.step;
-    if (q.step >= q.steps) q.done = 1;
-    return;
-  }
-  if (b >= W->npois) return;
-  Req &q = R[W->pois_slot[b]];
+// the (r, r) step of a request
+__device__ __forceinline__ void advance(Pois &q, double (*sh)[CTA_Y], int grp) {
   if (q.done) return;
   const int ph = q.phase;
-  const bool newstep = ph == 0 && q.newstep;  // uniform over the CTA
-  const double g = request_sum(q, 1, sh);
-  const double bb = newstep ? request_sum(q, 0, sh) : 0.0;
-  if (threadIdx.x != 0) return;
+  const bool newstep = ph == 0 && q.newstep;  // uniform over the group
+  const double g = request_sum(q, 1, sh, grp);
+  const double bb = newstep ? request_sum(q, 0, sh, grp) : 0.0;
+  if (threadIdx.x % GT != 0) return;
   if (ph == 0 || ph == 3) {  // g = (b - A x, b - A x) in FP64
     if (newstep) {  // heat: relative to the step's right-hand side
       q.rr0 = bb;
@@ -416,118 +423,279 @@ __global__ void __launch_bounds__(256) scalars_b(const Work *__restrict__ W, Req
   q.gamma = g;
 }
 
+// Grid barrier of a cooperative launch.  bar[0] counts arrivals for the
+// engine's life (`target` is its value, modulo 2^32, when all CTAs of this
+// barrier have arrived); the wait is bounded, and a CTA that gives up sets
+// bar[1], which makes every other one give up.  False in every thread when
+// the barrier failed.
+constexpr unsigned kSpin = 1u << 22;  // polls of some 0.5 us: seconds
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int *ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned seen, k = 0;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+    } while ((int)(seen - target) < 0 && ++k < kSpin);
+    bool good = (int)(seen - target) >= 0;
+    if (!good) atomicExch(bar + 1, 1u);
+    *ok = good;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+template <typename TI>
+__device__ __forceinline__ void pw_any(const Pois &q, int t, int g, double (*sh)[CTA_Y]) {
+  switch (q.ry) {  // uniform over the group
+    case 1: pw_tile<TI, 1>(q, t, g, sh); break;
+    case 2: pw_tile<TI, 2>(q, t, g, sh); break;
+    default: pw_tile<TI, 4>(q, t, g, sh);
+  }
+}
+template <typename TI>
+__device__ __forceinline__ void xr_any(const Pois &q, int t, int g, double (*sh)[CTA_Y]) {
+  switch (q.ry) {
+    case 1: xr_tile<TI, 1>(q, t, g, sh); break;
+    case 2: xr_tile<TI, 2>(q, t, g, sh); break;
+    default: xr_tile<TI, 4>(q, t, g, sh);
+  }
+}
+
+// `iters` iterations of every Poisson and heat request in one cooperative
+// launch of one CTA per SM.  CTA c owns tiles [c T / G, (c + 1) T / G) of the
+// work list's T, so it meets few requests; its groups take the tiles in turn.
+//
+// Latency-bound: the requests' vectors live in L2 and a 640^2 request's pass
+// is 1 to 2 us of work, so what counts is what lies between the passes: two
+// grid barriers per iteration in place of four kernel boundaries and two
+// one-CTA-per-request scalar kernels.
+//
+// Between the barriers a request's partial sums of column 0 (column 1) are
+// written by pw_tile (xr_tile) before, and read by form_alpha (advance)
+// after the barrier; the next write follows the next barrier.
+template <typename TI>
+__global__ void __launch_bounds__(GT * pois_groups<TI>(), 1) pois_iterate(
+    const Work *__restrict__ W, Req *R, int iters, unsigned *bar, unsigned base) {
+  constexpr int NG = pois_groups<TI>();
+  __shared__ double shs[NG][2][CTA_Y];
+  __shared__ int ok;
+  extern __shared__ Pois qs[];  // this CTA's requests
+  const int g = threadIdx.x / GT;
+  const long long total = W->pois_pref[W->npois];
+  const long long t0 = total * blockIdx.x / gridDim.x, t1 = total * (blockIdx.x + 1) / gridDim.x;
+  const int k0 = t1 > t0 ? find_req(W->pois_pref, W->npois, t0) : 0;
+  const int nk = t1 > t0 ? find_req(W->pois_pref, W->npois, t1 - 1) - k0 + 1 : 0;
+  for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+    const Req &r = R[W->pois_slot[k0 + k]];
+    Pois &q = qs[k];
+    q.kind = r.kind; q.n = r.n; q.pitch = r.pitch; q.tiles_x = r.tiles_x; q.tiles = r.tiles;
+    q.ry = r.ry; q.phase = r.phase; q.done = r.done; q.outer = r.outer; q.iters = r.iters;
+    q.step = r.step; q.par = r.par; q.newstep = r.newstep; q.max_inner = r.max_inner;
+    q.max_outer = r.max_outer; q.steps = r.steps; q.tol = r.tol; q.inner_tol = r.inner_tol;
+    q.diag = r.diag; q.off = r.off; q.alpha = r.alpha; q.beta = r.beta; q.gamma = r.gamma;
+    q.gamma_in0 = r.gamma_in0; q.rr0 = r.rr0; q.rel = r.rel; q.x = r.x; q.b = r.b;
+    q.part = r.part; q.r = r.r; q.w = r.w; q.p0 = r.p0; q.p1 = r.p1;
+  }
+  __syncthreads();
+  double(*sh)[CTA_Y] = shs[g];
+  for (int it = 0; it < iters; it++) {
+    for (long long u = t0 + g; u < t1; u += NG) {
+      const int k = nk == 1 ? k0 : find_req(W->pois_pref, W->npois, u);
+      const Pois &q = qs[k - k0];
+      if (!q.done && q.phase == 2) pw_any<TI>(q, (int)(u - W->pois_pref[k]), g, sh);
+    }
+    base += gridDim.x;
+    if (!grid_barrier(bar, base, &ok)) return;
+    for (int k = g; k < nk; k += NG) form_alpha(qs[k], sh, g);
+    __syncthreads();
+    for (long long u = t0 + g; u < t1; u += NG) {
+      const int k = nk == 1 ? k0 : find_req(W->pois_pref, W->npois, u);
+      const Pois &q = qs[k - k0];
+      if (!q.done) xr_any<TI>(q, (int)(u - W->pois_pref[k]), g, sh);
+    }
+    base += gridDim.x;
+    if (!grid_barrier(bar, base, &ok)) return;
+    for (int k = g; k < nk; k += NG) advance(qs[k], sh, g);
+    __syncthreads();
+  }
+  // the CTA with a request's first tile writes its state back
+  for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+    if (W->pois_pref[k0 + k] < t0) continue;
+    Req &r = R[W->pois_slot[k0 + k]];
+    const Pois &q = qs[k];
+    r.phase = q.phase; r.done = q.done; r.outer = q.outer; r.iters = q.iters; r.step = q.step;
+    r.par = q.par; r.newstep = q.newstep; r.alpha = q.alpha; r.beta = q.beta; r.gamma = q.gamma;
+    r.gamma_in0 = q.gamma_in0; r.rr0 = q.rr0; r.rel = q.rel;
+  }
+}
+
 // ---------------------------------------------------------------- ADI
-// grid of n^3 points including the Dirichlet boundary (adi/preproc_kernel.h)
+// grid of n^3 points including the Dirichlet boundary (adi/preproc_kernel.h):
+// a = c = -lambda / 2, b = 1 + lambda inside, identity rows on the boundary.
+// A line of n points is L lanes (Req::ry: 8, 16 or 32, the fewest that hold
+// it) with chunks of ADI_CL points in registers, the chunk ends solved among
+// the lanes (ob2_trid.cuh); a CTA of 256 threads is a unit of 256 / L lines.
+// One launch per direction: one thread per line and a sequential recurrence
+// took 80 to 130 us for seven requests of 32^3 to 160^3, too few threads to
+// cover its latency.
 
-__global__ void __launch_bounds__(256) adi_pre(const Work *__restrict__ W, Req *R) {
-  const long long total = W->pre_pref[W->nadi];
-  for (long long un = blockIdx.x; un < total; un += gridDim.x) {
-    const int k = find_req(W->pre_pref, W->nadi, un);
-    const Req &q = R[W->adi_slot[k]];
-    if (q.done) continue;
-    const int n = q.n;
-    const int t = (int)(un - W->pre_pref[k]);
-    const int tx = (n + 31) / 32, ty = (n + 7) / 8;
-    const int i = (t % tx) * 32 + threadIdx.x;
-    const int j = ((t / tx) % ty) * 8 + threadIdx.y;
-    const int z = t / (tx * ty);
-    if (i >= n || j >= n) continue;
-    const long long o = ((long long)z * n + j) * n + i;
-    const double *u = q.u;
-    double d = 0.0;
-    if (!(i == 0 || i == n - 1 || j == 0 || j == n - 1 || z == 0 || z == n - 1)) {
-      const long long sy = n, sz = (long long)n * n;
-      d = q.lambda * (u[o - 1] + u[o + 1] + u[o - sy] + u[o + sy] + u[o - sz] + u[o + sz] -
-                      6.0 * u[o]);
+// the chunk's coefficients (rows k0 .. of a line of n), then its end rows
+// reduced over the line's lanes: x_last of the chunk is D, its first is
+// returned in xf
+template <int L>
+__device__ __forceinline__ void adi_line(double (&a)[ADI_CL], double (&c)[ADI_CL],
+                                         double (&d)[ADI_CL], int k0, int n, bool edge,
+                                         double lambda) {
+  double b[ADI_CL];
+#pragma unroll
+  for (int i = 0; i < ADI_CL; i++) {
+    const int k = k0 + i;
+    const bool in = k > 0 && k < n - 1 && !edge;
+    a[i] = c[i] = in ? -0.5 * lambda : 0.0;
+    b[i] = in ? 1.0 + lambda : 1.0;
+  }
+  chunk_reduce<ADI_CL>(a, b, c, d);
+}
+
+// right-hand side lambda * (7-point Laplacian of u), then the x solve; the
+// solution in du
+template <int L>
+__device__ __forceinline__ void adi_x_unit(const Req &q, long long line) {
+  const int n = q.n, lane = threadIdx.x % L, k0 = lane * ADI_CL;
+  const bool active = line < (long long)n * n;
+  const int y = active ? (int)(line % n) : 0, z = active ? (int)(line / n) : 0;
+  const bool edge = y == 0 || y == n - 1 || z == 0 || z == n - 1;
+  const long long sy = n, sz = (long long)n * n, o = z * sz + y * sy + k0;
+  const double *u = q.u;
+  const bool whole = active && k0 + ADI_CL <= n;
+  double a[ADI_CL], c[ADI_CL], d[ADI_CL];
+  if (whole && !edge) {
+    double m[ADI_CL], n1[ADI_CL], n2[ADI_CL], n3[ADI_CL], n4[ADI_CL];
+    load_chunk<double, ADI_CL>(u + o, m);
+    load_chunk<double, ADI_CL>(u + o - sy, n1);
+    load_chunk<double, ADI_CL>(u + o + sy, n2);
+    load_chunk<double, ADI_CL>(u + o - sz, n3);
+    load_chunk<double, ADI_CL>(u + o + sz, n4);
+    const double lo = k0 > 0 ? u[o - 1] : 0.0, hi = k0 + ADI_CL < n ? u[o + ADI_CL] : 0.0;
+#pragma unroll
+    for (int i = 0; i < ADI_CL; i++) {
+      const double w = i > 0 ? m[i > 0 ? i - 1 : 0] : lo, e = i < ADI_CL - 1 ? m[i < ADI_CL - 1 ? i + 1 : 0] : hi;
+      d[i] = q.lambda * (w + e + n1[i] + n2[i] + n3[i] + n4[i] - 6.0 * m[i]);
+      if (k0 + i == 0 || k0 + i == n - 1) d[i] = 0.0;
     }
-    q.du[o] = d;
+  } else {
+#pragma unroll
+    for (int i = 0; i < ADI_CL; i++) {
+      const int k = k0 + i;
+      d[i] = 0.0;
+      if (active && !edge && k > 0 && k < n - 1)
+        d[i] = q.lambda * (u[o + i - 1] + u[o + i + 1] + u[o + i - sy] + u[o + i + sy] +
+                           u[o + i - sz] + u[o + i + sz] - 6.0 * u[o + i]);
+    }
+  }
+  adi_line<L>(a, c, d, k0, n, edge, q.lambda);
+  double A, C, xl;
+  group_reduce<L>(a[0], c[0], d[0], a[ADI_CL - 1], c[ADI_CL - 1], d[ADI_CL - 1], lane, A, C, xl);
+  double xp = __shfl_up_sync(0xffffffffu, xl, 1, L);
+  if (lane == 0) xp = 0.0;
+  const double xf = d[0] - a[0] * xp - c[0] * xl;
+  if (!active) return;
+#pragma unroll
+  for (int i = 0; i < ADI_CL; i++)
+    d[i] = i == 0 ? xf : i == ADI_CL - 1 ? xl : d[i] - a[i] * xf - c[i] * xl;
+  if (whole) {
+    store_chunk<double, ADI_CL>(q.du + o, d);
+  } else {
+#pragma unroll
+    for (int i = 0; i < ADI_CL; i++)
+      if (k0 + i < n) q.du[o + i] = d[i];
   }
 }
 
-// x solve: 32 lines of one z plane staged through shared memory
-__global__ void __launch_bounds__(128) adi_x(const Work *__restrict__ W, Req *R) {
-  extern __shared__ double sm[];  // [ADI_XL][n + 1]
-  const long long total = W->x_pref[W->nadi];
-  for (long long un = blockIdx.x; un < total; un += gridDim.x) {
-    const int k = find_req(W->x_pref, W->nadi, un);
-    const Req &q = R[W->adi_slot[k]];
-    if (q.done) continue;  // uniform over the CTA
-    const int n = q.n, ld = n + 1;
-    const int t = (int)(un - W->x_pref[k]);
-    const int nyb = (n + ADI_XL - 1) / ADI_XL;
-    const int y0 = (t % nyb) * ADI_XL, z = t / nyb;
-    double *du = q.du + (long long)z * n * n;
-    for (int e = threadIdx.x; e < ADI_XL * n; e += blockDim.x) {
-      const int l = e / n, xi = e - l * n;
-      if (y0 + l < n) sm[l * ld + xi] = du[(long long)(y0 + l) * n + xi];
-    }
-    __syncthreads();
-    if (threadIdx.x < ADI_XL && y0 + threadIdx.x < n) {
-      double *v = sm + threadIdx.x * ld;
-      const double a = q.a_coef;
-      double prev = v[0] * q.mm[0];
-      v[0] = prev;
-      for (int xi = 1; xi < n - 1; xi++) {
-        prev = (v[xi] - a * prev) * q.mm[xi];
-        v[xi] = prev;
-      }
-      v[n - 1] = v[n - 1] * q.mm[n - 1];  // Dirichlet row: a = 0
-      double nxt = v[n - 1];
-      for (int xi = n - 2; xi >= 0; xi--) {
-        nxt = v[xi] - q.cp[xi] * nxt;
-        v[xi] = nxt;
-      }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < ADI_XL * n; e += blockDim.x) {
-      const int l = e / n, xi = e - l * n;
-      if (y0 + l < n) du[(long long)(y0 + l) * n + xi] = sm[l * ld + xi];
-    }
-    __syncthreads();
+// y (DIR 1) or z (DIR 2) solve of 256 / L neighbouring lines in line-major
+// order (runs of 256 / L elements along x); z adds its solution into u
+template <int DIR, int L>
+__device__ __forceinline__ void adi_s_unit(const Req &q, long long line0, double *sm) {
+  constexpr int LPB = 256 / L, pitch = L + 1, field = LPB * pitch;
+  const int n = q.n, tid = threadIdx.x, p = tid / LPB, l = tid % LPB, k0 = p * ADI_CL;
+  const long long line = line0 + l, nn = (long long)n * n;
+  const bool active = line < nn;
+  const int x = active ? (int)(line % n) : 0, o = active ? (int)(line / n) : 0;  // o: z or y
+  const bool edge = x == 0 || x == n - 1 || o == 0 || o == n - 1;
+  const long long s = DIR == 1 ? n : nn;
+  const long long base = (DIR == 1 ? o * nn : (long long)o * n) + x + k0 * s;
+  const double *src = q.du;
+  double a[ADI_CL], c[ADI_CL], d[ADI_CL];
+#pragma unroll
+  for (int i = 0; i < ADI_CL; i++) d[i] = active && k0 + i < n ? src[base + i * s] : 0.0;
+  adi_line<L>(a, c, d, k0, n, edge, q.lambda);
+  {
+    double *e = sm + l * pitch + p;
+    e[0] = a[0]; e[field] = c[0]; e[2 * field] = d[0];
+    e[3 * field] = a[ADI_CL - 1]; e[4 * field] = c[ADI_CL - 1]; e[5 * field] = d[ADI_CL - 1];
   }
+  __syncthreads();
+  {
+    const int lane = tid % L;
+    double *e = sm + (tid / L) * pitch + lane;
+    const double a0 = e[0], c0 = e[field], d0 = e[2 * field];
+    double A, C, xl;
+    group_reduce<L>(a0, c0, d0, e[3 * field], e[4 * field], e[5 * field], lane, A, C, xl);
+    double xp = __shfl_up_sync(0xffffffffu, xl, 1, L);
+    if (lane == 0) xp = 0.0;
+    e[2 * field] = d0 - a0 * xp - c0 * xl;  // this lane's own slots
+    e[5 * field] = xl;
+  }
+  __syncthreads();
+  const double xf = sm[2 * field + l * pitch + p], xl = sm[5 * field + l * pitch + p];
+  __syncthreads();  // the next unit overwrites the slots
+  if (!active) return;
+#pragma unroll
+  for (int i = 0; i < ADI_CL; i++)
+    if (k0 + i < n) {
+      const double v = i == 0 ? xf : i == ADI_CL - 1 ? xl : d[i] - a[i] * xf - c[i] * xl;
+      if (DIR == 2)
+        q.u[base + i * s] = q.u[base + i * s] + v;
+      else
+        q.du[base + i * s] = v;
+    }
 }
 
-// y (dir 1) or z (dir 2) solve: one thread per line, neighbouring threads on
-// neighbouring x (coalesced); the z solve adds its solution into u
+// solve along DIR (0 x, 1 y, 2 z) of every ADI request that has a step left
+// after `it` more steps than its count
 template <int DIR>
-__global__ void __launch_bounds__(32 * ADI_YZ) adi_yz(const Work *__restrict__ W, Req *R) {
-  const long long total = W->yz_pref[W->nadi];
+__global__ void __launch_bounds__(256, 3) adi_solve(const Work *__restrict__ W, Req *R, int it) {
+  __shared__ double sm[DIR ? 6 * (256 + 32) : 1];
+  const long long total = W->adi_pref[W->nadi];
   for (long long un = blockIdx.x; un < total; un += gridDim.x) {
-    const int k = find_req(W->yz_pref, W->nadi, un);
+    const int k = find_req(W->adi_pref, W->nadi, un);
     const Req &q = R[W->adi_slot[k]];
-    if (q.done) continue;
-    const int n = q.n;
-    const int t = (int)(un - W->yz_pref[k]);
-    const int nxb = (n + 31) / 32;
-    const int i = (t % nxb) * 32 + threadIdx.x;
-    const int c = (t / nxb) * ADI_YZ + threadIdx.y;  // the other coordinate
-    if (i >= n || c >= n) continue;
-    const long long s = DIR == 1 ? (long long)n : (long long)n * n;
-    const long long base = DIR == 1 ? (long long)c * n * n + i : (long long)c * n + i;
-    double *v = q.du + base;
-    const double a = q.a_coef;
-    double prev = v[0] * q.mm[0];
-    v[0] = prev;
-    for (int m = 1; m < n - 1; m++) {
-      prev = (v[m * s] - a * prev) * q.mm[m];
-      v[m * s] = prev;
-    }
-    v[(n - 1) * s] = v[(n - 1) * s] * q.mm[n - 1];  // Dirichlet row: a = 0
-    double nxt = v[(n - 1) * s];
-    if (DIR == 2) {
-      double *u = q.u + base;
-      u[(n - 1) * s] = u[(n - 1) * s] + nxt;
-      for (int m = n - 2; m >= 0; m--) {
-        nxt = v[m * s] - q.cp[m] * nxt;
-        u[m * s] = u[m * s] + nxt;
-      }
+    if (q.step + it >= q.steps) continue;  // uniform over the CTA
+    const int L = q.ry;
+    const long long line0 = (un - W->adi_pref[k]) * (256 / L);
+    if (DIR == 0) {
+      const long long line = line0 + threadIdx.x / L;
+      if (L == 8) adi_x_unit<8>(q, line);
+      else if (L == 16) adi_x_unit<16>(q, line);
+      else adi_x_unit<32>(q, line);
     } else {
-      for (int m = n - 2; m >= 0; m--) {
-        nxt = v[m * s] - q.cp[m] * nxt;
-        v[m * s] = nxt;
-      }
+      constexpr int D = DIR ? DIR : 1;
+      if (L == 8) adi_s_unit<D, 8>(q, line0, sm);
+      else if (L == 16) adi_s_unit<D, 16>(q, line0, sm);
+      else adi_s_unit<D, 32>(q, line0, sm);
     }
   }
+}
+
+// the step counts after `steps` steps of each request (or all it had left)
+__global__ void adi_count(const Work *__restrict__ W, Req *R, int steps) {
+  const int k = threadIdx.x;
+  if (k >= W->nadi) return;
+  Req &q = R[W->adi_slot[k]];
+  q.step = min(q.step + steps, q.steps);
+  q.iters = q.step;
+  if (q.step >= q.steps) q.done = 1;
 }
 
 // ---------------------------------------------------------------- init
@@ -598,19 +766,16 @@ struct ob2s_engine {
   int sms;
   Req *R_d;
   Work *W_d;
-  std::vector<Req> R;       // host copy (refreshed after every run)
+  Req *R;                   // host copy, pinned (refreshed after every run); slot MAXA
+                            // holds the grid barrier's words
   std::vector<int> used;    // slot in use
   std::vector<int> active;  // slot is in the work list
   std::vector<int> reported;
   std::vector<void *> mem;  // per slot allocation
   std::vector<size_t> bytes;
   bool work_dirty;
-  int pois_ctas_per_sm;  // resident CTAs per SM of the Poisson kernels
-  struct Graph {
-    int iters, variant, kernels;
-    cudaGraphExec_t exec;
-  };
-  std::vector<Graph> graphs;
+  unsigned *bar_d;     // grid barrier of pois_iterate (arrivals, failure), in R_d's last slot
+  unsigned bar_base;   // arrivals before the next launch
   long long launches;
   // the requests' memory: a pool of the engine's own that keeps freed
   // memory mapped (a request admitted after another retired reuses its
@@ -632,40 +797,32 @@ OB2_API size_t ob2s_request_bytes(int mode, int kind, int n) {
   return (size_t)n * n * n * 16 + (size_t)n * 16 + 4096;
 }
 
-// one engine iteration; the kernels of a request kind with no active
-// request are left out (variant bit 0: Poisson, bit 1: ADI)
-template <typename TI, int RY>
-static int launch_iteration(ob2s_engine *e, int variant) {
-  int k = 0;
-  if (variant & 1) {
-    const int g = e->sms * e->pois_ctas_per_sm;
-    pois_pw<TI, RY><<<g, dim3(TX, CTA_Y), 0, e->st>>>(e->W_d, e->R_d);
-    scalars_a<<<MAXA, 256, 0, e->st>>>(e->W_d, e->R_d);
-    pois_xr<TI, RY><<<g, dim3(TX, CTA_Y), 0, e->st>>>(e->W_d, e->R_d);
-    k += 3;
-  }
-  if (variant & 2) {
-    adi_pre<<<e->sms * 8, dim3(32, 8), 0, e->st>>>(e->W_d, e->R_d);
-    const size_t xsm = (size_t)ADI_XL * (ADI_MAX_N + 1) * sizeof(double);
-    adi_x<<<e->sms * 4, 128, xsm, e->st>>>(e->W_d, e->R_d);
-    adi_yz<1><<<e->sms * 16, dim3(32, ADI_YZ), 0, e->st>>>(e->W_d, e->R_d);
-    adi_yz<2><<<e->sms * 16, dim3(32, ADI_YZ), 0, e->st>>>(e->W_d, e->R_d);
-    k += 4;
-  }
-  scalars_b<<<2 * MAXA, 256, 0, e->st>>>(e->W_d, e->R_d);
-  return k + 1;
+static size_t pois_smem() { return sizeof(Pois) * MAXA; }
+
+// `iters` iterations of the Poisson and heat requests
+static cudaError_t launch_pois(ob2s_engine *e, int iters) {
+  void *args[] = {&e->W_d, &e->R_d, &iters, &e->bar_d, &e->bar_base};
+  const bool mixed = e->mode == OB2S_MIXED;
+  const void *f = mixed ? (const void *)pois_iterate<float> : (const void *)pois_iterate<double>;
+  const int threads = GT * (mixed ? pois_groups<float>() : pois_groups<double>());
+  const cudaError_t err =
+      cudaLaunchCooperativeKernel(f, dim3(e->sms), dim3(threads), args, pois_smem(), e->st);
+  if (err != cudaSuccess) return err;
+  e->bar_base += 2u * (unsigned)iters * (unsigned)e->sms;
+  e->launches++;
+  return cudaSuccess;
 }
 
-static int launch_iteration_any(ob2s_engine *e, int variant) {
-  const bool mixed = e->mode == OB2S_MIXED;
-  switch (e->tile_y) {  // tile height = 8 rows per thread
-    case 8:
-      return mixed ? launch_iteration<float, 1>(e, variant) : launch_iteration<double, 1>(e, variant);
-    case 16:
-      return mixed ? launch_iteration<float, 2>(e, variant) : launch_iteration<double, 2>(e, variant);
-    default:
-      return mixed ? launch_iteration<float, 4>(e, variant) : launch_iteration<double, 4>(e, variant);
+// `steps` steps of the ADI requests
+static cudaError_t launch_adi(ob2s_engine *e, int steps) {
+  for (int i = 0; i < steps; i++) {
+    adi_solve<0><<<e->sms * 6, 256, 0, e->st>>>(e->W_d, e->R_d, i);
+    adi_solve<1><<<e->sms * 6, 256, 0, e->st>>>(e->W_d, e->R_d, i);
+    adi_solve<2><<<e->sms * 6, 256, 0, e->st>>>(e->W_d, e->R_d, i);
   }
+  adi_count<<<1, MAXA, 0, e->st>>>(e->W_d, e->R_d, steps);
+  e->launches += 3LL * steps + 1;
+  return cudaGetLastError();
 }
 
 OB2_API int ob2s_create(ob2s_engine **out, int mode, double tol, double inner_tol, int max_inner,
@@ -684,40 +841,20 @@ OB2_API int ob2s_create(ob2s_engine **out, int mode, double tol, double inner_to
   e->max_inner = max_inner > 0 ? max_inner : 100000;
   cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, dev);
   if ((err = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking)) != cudaSuccess ||
-      (err = cudaMalloc(&e->R_d, sizeof(Req) * MAXA)) != cudaSuccess ||
+      (err = cudaMalloc(&e->R_d, sizeof(Req) * (MAXA + 1))) != cudaSuccess ||
+      (err = cudaMallocHost(&e->R, sizeof(Req) * (MAXA + 1))) != cudaSuccess ||
       (err = cudaMalloc(&e->W_d, sizeof(Work))) != cudaSuccess ||
-      (err = cudaMemset(e->R_d, 0, sizeof(Req) * MAXA)) != cudaSuccess ||
+      (err = cudaMemset(e->R_d, 0, sizeof(Req) * (MAXA + 1))) != cudaSuccess ||
       (err = cudaMemset(e->W_d, 0, sizeof(Work))) != cudaSuccess ||
-      (err = cudaFuncSetAttribute(adi_x, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(ADI_XL * (ADI_MAX_N + 1) * sizeof(double)))) !=
-          cudaSuccess) {
+      (err = cudaFuncSetAttribute(mode == OB2S_MIXED ? (const void *)pois_iterate<float>
+                                                     : (const void *)pois_iterate<double>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)pois_smem())) != cudaSuccess) {
     delete e;
     return rc(err);
   }
-  {
-    // persistent grids: as many CTAs as can be resident at once
-    int nb = 0, nb2 = 0;
-    const bool mixed = mode == OB2S_MIXED;
-    auto occ = [&](const void *f) {
-      int b = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, TX * CTA_Y, 0);
-      return b;
-    };
-    switch (tile_y) {
-      case 8:
-        nb = occ(mixed ? (const void *)pois_pw<float, 1> : (const void *)pois_pw<double, 1>);
-        nb2 = occ(mixed ? (const void *)pois_xr<float, 1> : (const void *)pois_xr<double, 1>);
-        break;
-      case 16:
-        nb = occ(mixed ? (const void *)pois_pw<float, 2> : (const void *)pois_pw<double, 2>);
-        nb2 = occ(mixed ? (const void *)pois_xr<float, 2> : (const void *)pois_xr<double, 2>);
-        break;
-      default:
-        nb = occ(mixed ? (const void *)pois_pw<float, 4> : (const void *)pois_pw<double, 4>);
-        nb2 = occ(mixed ? (const void *)pois_xr<float, 4> : (const void *)pois_xr<double, 4>);
-    }
-    e->pois_ctas_per_sm = std::max(1, std::min(nb, nb2));
-  }
+  e->bar_d = (unsigned *)(e->R_d + MAXA);
+  e->bar_base = 0;
   {
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
@@ -729,6 +866,7 @@ OB2_API int ob2s_create(ob2s_engine **out, int mode, double tol, double inner_to
       cudaStreamDestroy(e->st);
       cudaFree(e->R_d);
       cudaFree(e->W_d);
+      cudaFreeHost(e->R);
       delete e;
       return rc(err);
     }
@@ -738,12 +876,12 @@ OB2_API int ob2s_create(ob2s_engine **out, int mode, double tol, double inner_to
       cudaStreamDestroy(e->st);
       cudaFree(e->R_d);
       cudaFree(e->W_d);
+      cudaFreeHost(e->R);
       delete e;
       return rc(err);
     }
   }
-  e->R.assign(MAXA, Req());
-  memset(e->R.data(), 0, sizeof(Req) * MAXA);
+  memset(e->R, 0, sizeof(Req) * (MAXA + 1));
   e->used.assign(MAXA, 0);
   e->active.assign(MAXA, 0);
   e->reported.assign(MAXA, 0);
@@ -772,34 +910,16 @@ OB2_API int ob2s_reserve(ob2s_engine *e, size_t bytes) {
 OB2_API void ob2s_destroy(ob2s_engine *e) {
   if (!e) return;
   cudaStreamSynchronize(e->st);
-  for (auto &g : e->graphs) cudaGraphExecDestroy(g.exec);
   for (int k = 0; k < MAXA; k++)
     if (e->mem[k]) cudaFreeAsync(e->mem[k], e->st);
   cudaStreamSynchronize(e->st);
   cudaFree(e->R_d);
   cudaFree(e->W_d);
+  cudaFreeHost(e->R);
   cudaFree(e->sum_d);
   cudaMemPoolDestroy(e->pool);
   cudaStreamDestroy(e->st);
   delete e;
-}
-
-static void host_thomas_coefs(int n, double lambda, std::vector<double> &cp,
-                              std::vector<double> &mm, double *a_out) {
-  // rows 0 and n-1: identity (Dirichlet); interior: a = c = -lambda/2,
-  // b = 1 + lambda (adi/preproc_kernel.h).  c'_i and 1/(b_i - a_i c'_{i-1}).
-  const double a = -0.5 * lambda, b = 1.0 + lambda, c = -0.5 * lambda;
-  cp.assign(n, 0.0);
-  mm.assign(n, 0.0);
-  mm[0] = 1.0;
-  cp[0] = 0.0;
-  for (int i = 1; i < n; i++) {
-    const bool edge = i == n - 1;
-    const double ai = edge ? 0.0 : a, bi = edge ? 1.0 : b, ci = edge ? 0.0 : c;
-    mm[i] = 1.0 / (bi - ai * cp[i - 1]);
-    cp[i] = ci * mm[i];
-  }
-  *a_out = a;
 }
 
 OB2_API int ob2s_submit(ob2s_engine *e, int kind, int n, int seed, int steps, int *id) {
@@ -835,6 +955,7 @@ OB2_API int ob2s_submit(ob2s_engine *e, int kind, int n, int seed, int steps, in
   if (grid2d) {
     q.pitch = (n + 4) & ~1;  // even, >= n + 3: columns 0 .. n + C0
     q.tiles_x = (n + TXC - 1) / TXC;
+    q.ry = e->tile_y / CTA_Y;
     q.tiles = q.tiles_x * ((n + e->tile_y - 1) / e->tile_y);
     const size_t p = (size_t)q.pitch * (n + 2);
     const size_t ei = elem_inner(e->mode);
@@ -860,8 +981,7 @@ OB2_API int ob2s_submit(ob2s_engine *e, int kind, int n, int seed, int steps, in
   } else {
     q.u = (double *)take((size_t)n * n * n * 8);
     q.du = (double *)take((size_t)n * n * n * 8);
-    q.cp = (double *)take((size_t)n * 8);
-    q.mm = (double *)take((size_t)n * 8);
+    q.ry = n <= 8 * ADI_CL ? 8 : n <= 16 * ADI_CL ? 16 : 32;
   }
   if ((size_t)(c - (char *)m) > nb) {  // cannot happen: the slack covers the rounding
     cudaFreeAsync(m, e->st);
@@ -874,14 +994,7 @@ OB2_API int ob2s_submit(ob2s_engine *e, int kind, int n, int seed, int steps, in
   } else {
     q.lambda = 1.0;
     q.steps = steps;
-    std::vector<double> cp, mm;
-    host_thomas_coefs(n, q.lambda, cp, mm, &q.a_coef);
-    cudaMemcpyAsync(q.cp, cp.data(), (size_t)n * 8, cudaMemcpyHostToDevice, e->st);
-    cudaMemcpyAsync(q.mm, mm.data(), (size_t)n * 8, cudaMemcpyHostToDevice, e->st);
     adi_init<<<dim3((n + 127) / 128, n, n), 128, 0, e->st>>>(q.u, n, seed);
-    // the coefficient tables are copied from host vectors that go out of
-    // scope: wait for them
-    cudaStreamSynchronize(e->st);
   }
   err = cudaMemcpyAsync(e->R_d + slot, &q, sizeof(Req), cudaMemcpyHostToDevice, e->st);
   if (err == cudaSuccess) err = cudaStreamSynchronize(e->st);
@@ -916,9 +1029,8 @@ static int upload_work(ob2s_engine *e) {
       const int n = q.n;
       const int a = w.nadi;
       w.adi_slot[a] = k;
-      w.pre_pref[a + 1] = w.pre_pref[a] + (long long)((n + 31) / 32) * ((n + 7) / 8) * n;
-      w.x_pref[a + 1] = w.x_pref[a] + (long long)((n + ADI_XL - 1) / ADI_XL) * n;
-      w.yz_pref[a + 1] = w.yz_pref[a] + (long long)((n + 31) / 32) * ((n + ADI_YZ - 1) / ADI_YZ);
+      const int lpu = 256 / q.ry;  // lines per unit
+      w.adi_pref[a + 1] = w.adi_pref[a] + ((long long)n * n + lpu - 1) / lpu;
       w.nadi++;
     }
   }
@@ -933,36 +1045,29 @@ OB2_API int ob2s_run(ob2s_engine *e, int iters, int *ids, int cap, int *n_done) 
   *n_done = 0;
   int err;
   if (e->work_dirty && (err = upload_work(e))) return err;
-  int variant = 0;
-  for (int k = 0; k < MAXA; k++)
-    if (e->active[k]) variant |= e->R[k].kind != OB2S_ADI3D ? 1 : 2;
-  if (variant) {
-    ob2s_engine::Graph *gr = nullptr;
-    for (auto &g : e->graphs)
-      if (g.iters == iters && g.variant == variant) gr = &g;
-    if (!gr) {
-      cudaGraph_t graph;
-      cudaGraphExec_t ge = nullptr;
-      cudaError_t ce = cudaStreamBeginCapture(e->st, cudaStreamCaptureModeThreadLocal);
-      if (ce != cudaSuccess) return rc(ce);
-      int kernels = 0;
-      for (int i = 0; i < iters; i++) kernels += launch_iteration_any(e, variant);
-      ce = cudaStreamEndCapture(e->st, &graph);
-      if (ce != cudaSuccess) return rc(ce);
-      ce = cudaGraphInstantiate(&ge, graph, 0);
-      cudaGraphDestroy(graph);
-      if (ce != cudaSuccess) return rc(ce);
-      e->graphs.push_back({iters, variant, kernels, ge});
-      gr = &e->graphs.back();
-    }
-    cudaError_t ce = cudaGraphLaunch(gr->exec, e->st);
-    if (ce != cudaSuccess) return rc(ce);
-    e->launches += gr->kernels;
+  bool pois = false;
+  int adi = 0;  // most steps that an ADI request has left
+  for (int k = 0; k < MAXA; k++) {
+    if (!e->active[k]) continue;
+    if (e->R[k].kind != OB2S_ADI3D)
+      pois = true;
+    else
+      adi = std::max(adi, e->R[k].steps - e->R[k].step);
   }
-  cudaError_t ce = cudaMemcpyAsync(e->R.data(), e->R_d, sizeof(Req) * MAXA,
-                                   cudaMemcpyDeviceToHost, e->st);
+  if (pois) {
+    const cudaError_t ce = launch_pois(e, iters);
+    if (ce != cudaSuccess) return rc(ce);
+  }
+  if (adi) {
+    const cudaError_t ce = launch_adi(e, std::min(adi, iters));
+    if (ce != cudaSuccess) return rc(ce);
+  }
+  cudaError_t ce = cudaMemcpyAsync(e->R, e->R_d, sizeof(Req) * (MAXA + 1), cudaMemcpyDeviceToHost,
+                                   e->st);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
   if (ce != cudaSuccess) return rc(ce);
+  if (((const unsigned *)(e->R + MAXA))[1])  // a grid barrier gave up
+    return (int)cudaErrorLaunchTimeout;
   for (int k = 0; k < MAXA; k++) {
     if (!e->used[k] || !e->R[k].done) continue;
     if (e->active[k]) {
