@@ -191,14 +191,15 @@ OPS_API void ob2_flush(void);
 OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int dim,
                            const int *range, ops_arg *args, int nargs);
 OPS_API void ob2_loop_end(ob2_loop *L);
-/* Grid of a reduction loop whose threads take up to max_rows consecutive
- * rows of a tile: *rows = max_rows when tiles of that height fill a wave of
- * CTAs (`resident` per SM, times OPS_B200_RED_WAVES), else 1; tiles[0..2] =
- * tiles of L->block along x, y (block[1] * rows rows) and z (the folded 3rd
- * to 5th axes).  Returns the CTAs: one wave at most, evened out over the
- * trips; L->partials is made large enough for them. */
-OPS_API unsigned ob2_red_grid(ob2_loop *L, int max_rows, int resident, unsigned tiles[3],
-                              int *rows);
+/* Grid of a reduction loop whose threads take *cols columns (block[0] apart)
+ * and *rows consecutive rows of a tile; both are set to 1 where tiles of that
+ * size do not fill half a wave of CTAs (`resident` per SM, times
+ * OPS_B200_RED_WAVES).  tiles[0..2] = tiles of L->block along x (block[0] *
+ * cols columns), y (block[1] * rows rows) and z (the folded 3rd to 5th axes).
+ * Returns the CTAs: one wave at most, evened out over the trips; L->partials
+ * is made large enough for them. */
+OPS_API unsigned ob2_red_grid(ob2_loop *L, int *cols, int *rows, int resident,
+                              unsigned tiles[3]);
 /* 1 when some dat is passed more than once and written through one of the
  * arguments: the loop's kernel must then not assume its dat pointers are
  * unaliased. */

@@ -249,7 +249,7 @@ OB2_API int ob2_halo_run_noalloc(const ob2_halo_task *tasks_host, int ntasks) {
 // LR lanes (the smallest power of two that covers a row, at most a warp)
 // copies a row, or a piece of kPiece units of a long one, with four accesses
 // per lane in flight and one division per row; a 187 x 180 x 139 box of 3
-// FP64 components (112 MB each way) takes 36 us against 64 us for one
+// FP64 components (112 MB each way) takes 39 us against 64 us for one
 // element per thread with two 64-bit divisions and a component loop.
 // Components of a SoA dat lie apart: each is a box of its own (STR) whose
 // buffer elements are nc apart.

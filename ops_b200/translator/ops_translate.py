@@ -327,6 +327,11 @@ class Translator:
         # rows per thread and tile of a reduction kernel (0: by red_rows)
         self.rpy = max(0, int(os.environ.get("OPS_B200_RPY", "0")))
         self.light_max = int(os.environ.get("OPS_B200_LIGHT", "4"))
+        # common-layout kernels (emit_uni): columns and rows per thread (0: by
+        # uni_shape), resident CTAs of 512 threads per SM
+        self.upx = max(0, int(os.environ.get("OPS_B200_UPX", "0")))
+        self.upy = max(0, int(os.environ.get("OPS_B200_UPY", "0")))
+        self.uminb = max(0, int(os.environ.get("OPS_B200_UMINB", "0")))
         # OPS_B200_CHECK=1: OPS_ACCn accesses are checked against their dat's
         # allocation; an access outside it prints its kernel, argument, point
         # and offset (device printf) and is redirected to the dat's first
@@ -710,8 +715,8 @@ class Translator:
         w("  const unsigned bx = loc - r * f.gx[i], by = r % f.gy[i], bz = r / f.gy[i];")
         w("  const char *prm = f.blob + f.off[i];")
         w("  switch (f.id[i]) {")
-        for k, (P, BF) in enumerate(items):
-            w("    case %d: %s<false, IDX32>(*(const %s *)prm, bx, by, bz); break;" % (k, BF, P))
+        for k, (P, body) in enumerate(items):
+            w("    case %d: %s(*(const %s *)prm, bx, by, bz); break;" % (k, body, P))
         w("    default: break;")
         w("  }")
         w("}")
@@ -773,6 +778,179 @@ class Translator:
         widest = max([self.ELEM_BYTES.get(p.base_type, 8) for i, a, p in dats] or [8])
         return base * max(1, 8 // widest)
 
+    def uni_dats(self, loop: Loop, dats):
+        """True when a loop can have a common-layout kernel: up to 3D, ACC
+        parameters, every dat of one component, none optional or prolong."""
+        return (loop.ndim <= 3 and not self.check and len(dats) > 0 and
+                all(p.is_acc and a.dim.strip() == "1" and not a.opt and not a.prolong
+                    for i, a, p in dats))
+
+    def light_arithmetic(self, kd) -> bool:
+        """True for a short kernel body (as light_y_stencil) without
+        divisions, square roots and the like: several points of a thread
+        then fit the registers."""
+        body = mask_comments_strings(kd.text[kd.text.find("{"):])
+        return body.count(";") <= self.light_max and \
+            re.search(r"/|\b(?:::ob2::div|sqrt|cbrt|exp|log|pow|sin|cos|tan|atan2?|hypot)f?\s*\(",
+                      body) is None
+
+    def uni_shape(self, loop: Loop, kd, dats, reds):
+        """(columns, rows) per thread of a loop's common-layout kernel.
+        Measured on one B200 against the general kernel (us, 4096^2 and
+        3840^2): copy 69.6 -> 36, p = r + b p 75.4 -> 58.7, flux update 282 ->
+        265 and 5-point sweep 61.5 -> 58.0 FP64, 38.2 -> 36.5 FP32 with 4
+        columns; loops with divisions or square roots lose with more than one
+        (equation of state 122 -> 150, y flux 238 -> 372).  3D 7-point sweep
+        384 x 300 x 280 FP64: 2 rows 136, 2 columns 140 to 187, 1 row 150."""
+        if reds:
+            # a dat that is read and written: the compiler may hoist the next
+            # point's load above this point's store only along x, where the
+            # points lie a constant apart (mixed CG update at 4096^2: 4 rows
+            # 113 us, 4 columns 104)
+            rr = self.red_rows(dats)
+            rw = any(a.acc == "OPS_RW" for i, a, p in dats)
+            return (rr, 1) if rw and self.light_arithmetic(kd) else (1, rr)
+        px, py = 1, 1
+        widest = max(self.ELEM_BYTES.get(p.base_type, 8) for i, a, p in dats)
+        if self.light_y_stencil(kd):
+            py = 2 * max(1, 8 // widest)
+        if loop.ndim < 3 and self.light_arithmetic(kd):
+            px = 4
+        return self.upx or px, self.upy or py
+
+    def emit_uni(self, loop: Loop, kd, P, base, dats, reds, px, py, aw, w) -> None:
+        """The common-layout kernel of a loop: every dat argument has unit x
+        stride and the same row and plane strides (the usual case: dats of
+        one block, stencils without strides; checked by the stub), so one
+        element offset per point serves all of them.  A thread covers px
+        columns 32 apart and py consecutive rows; the tile function takes the
+        dats as __restrict__ pointers, so that the loads of all its points can
+        be issued before the first store, and walks the rows by pointer, so
+        that rows shared by the stencil are loaded once."""
+        ey, ez = "p.ey%d" % dats[0][0], "p.ez%d" % dats[0][0]
+        es = [p.base_type for i, a, p in dats]
+        rprm = "".join(", %s *red%d" % (p.base_type, i) for i, a, p in reds)
+        rcall = "".join(", red%d" % i for i, a, p in reds)
+        off = "x" + (" + %s * %s" % ("y", ey) if loop.ndim > 1 else "") + \
+            (" + z * %s" % ez if loop.ndim > 2 else "")
+        w("static __device__ __forceinline__ void ob2u_%s(const %s &p, int x, int y, int z%s%s) {" %
+          (base, P, "".join(", %s *c%d" % (p.base_type, i) for i, a, p in dats), rprm))
+        call = []
+        for i, (a, pr) in enumerate(zip(loop.args, kd.params)):
+            if a.kind == "dat":
+                w("  ACC<%s> a%d(c%d, 1, %s, %s, p.ed%d);" % (pr.base_type, i, i, ey, ez, i))
+                call.append("a%d" % i)
+            elif a.kind == "gbl":
+                call.append("(%s *)p.g%d" % (pr.base_type, i))
+            elif a.kind == "reduce":
+                call.append("red%d" % i)
+            elif a.kind == "idx":
+                call.append("idx")
+        if any(a.kind == "idx" for a in loop.args):
+            w("  int idx[3] = {x, y, z};")
+        w("  %s(%s);" % (loop.kernel, ", ".join(call)))
+        w("}")
+        for variant, qual in (("R", "__restrict__ "), ("A", "")):
+            w("static __device__ __forceinline__ void ob2ut_%s_%s(const %s &p, int x, int y, int z%s%s) {" %
+              (base, variant, P, "".join(", %s *%sq%d" % (pr.base_type, qual, i)
+                                         for i, a, pr in dats), rprm))
+            w("  const long long r = %s;" % (ey if loop.ndim > 1 else "0"))
+            for i, a, pr in dats:
+                w("  %s *c%d = q%d + (%s);" % (pr.base_type, i, i, off))
+            w("#pragma unroll")
+            w("  for (int j = 0; j < %d; j++) {" % py)
+            w("#pragma unroll")
+            w("    for (int k = 0; k < %d; k++)" % px)
+            w("      ob2u_%s(p, x + 32 * k, y + j, z%s%s);" %
+              (base, "".join(", c%d + 32 * k" % i for i, a, pr in dats), rcall))
+            w("    " + " ".join("c%d += r;" % i for i, a, pr in dats))
+            w("  }")
+            w("}")
+        # tile at (x, y0): whole, or point by point at the range's edge
+        bs = "".join(", p.b%d" % i for i, a, pr in dats)
+        cs = "".join(", p.b%d + o" % i for i, a, pr in dats)
+        lo = "x >= p.lo0 && " if aw is not None else ""
+        rows = "p.rows" if reds else str(py)
+        cols = "blockDim.x * p.cols" if reds else str(32 * px)
+        full = "%sx + %d < p.hi0 && y0 + %d < p.hi1" % (lo, 32 * (px - 1), py - 1)
+        if reds:
+            full += " && p.rows == %d && p.cols == %d" % (py, px)
+        w("template <bool RESTRICT>")
+        w("static __device__ __forceinline__ void ob2ue_%s(const %s &p, int x, int y0, int z%s) {" %
+          (base, P, rprm))
+        w("  if (%s) {" % full)
+        w("    if (RESTRICT) ob2ut_%s_R(p, x, y0, z%s%s);" % (base, bs, rcall))
+        w("    else ob2ut_%s_A(p, x, y0, z%s%s);" % (base, bs, rcall))
+        w("  } else {")
+        w("    for (int y = y0; y < min(y0 + %s, p.hi1); y++)" % rows)
+        if px > 1:
+            w("      for (int xx = x; xx < min(x + (int)(%s), p.hi0); xx += 32) {" % cols)
+        else:
+            w("      for (int xx = x; xx < min(x + 1, p.hi0); xx++) {")
+        if aw is not None:
+            w("        if (xx < p.lo0) continue;")
+        w("        const int o = %s;" % re.sub(r"\bx\b", "xx", off, count=1))
+        w("        ob2u_%s(p, xx, y, z%s%s);" % (base, cs, rcall))
+        w("      }")
+        w("  }")
+        w("}")
+        if reds:
+            return
+        lb = "512, %d" % (self.uminb or (2 if px > 1 else 4))
+        w("template <bool RESTRICT>")
+        w("static __device__ __forceinline__ void ob2ub_%s(const %s &p, unsigned bx, unsigned by,"
+          " unsigned bz%s) {" % (base, P, ", bool align = true" if aw is not None else ""))
+        w("  const int y0 = p.lo1 + (int)(by * blockDim.y + threadIdx.y) * %d;" % py)
+        w("  const int z = p.lo2 + (int)(bz * blockDim.z + threadIdx.z);")
+        if aw is not None:
+            e = self.ELEM_BYTES[kd.params[aw].base_type]
+            w("  const int sh = align ? (int)(((unsigned long long)(p.b%d + (long long)p.lo0 +"
+              " (long long)y0 * %s + (long long)z * %s) / %d) & %d) : 0;" %
+              (aw, ey, ez, e, 128 // e - 1))
+        w("  const int x = p.lo0%s + (int)(bx * (blockDim.x * %d) + threadIdx.x);" %
+          (" - sh" if aw is not None else "", px))
+        w("  if (z < p.hi2) ob2ue_%s<RESTRICT>(p, x, y0, z);" % base)
+        w("}")
+        K = "ob2k_" + base
+        w("__global__ void __launch_bounds__(%s) %sU(const __grid_constant__ %s p) {" % (lb, K, P))
+        w("  ob2ub_%s<true>(p, blockIdx.x, blockIdx.y, blockIdx.z);" % base)
+        w("}")
+        w("__global__ void __launch_bounds__(%s) %sUM(const __grid_constant__ %sM m) {" % (lb, K, P))
+        w("  const unsigned it = blockIdx.z / m.gz;")
+        w("  ob2ub_%s<true>(m.p[it], blockIdx.x, blockIdx.y, blockIdx.z - it * m.gz);" % base)
+        w("}")
+        w("__global__ void __launch_bounds__(%s) %sUH(const __grid_constant__ %sM m,"
+          " const __grid_constant__ ob2_hfuse h) {" % (lb, K, P))
+        w("  const unsigned it = blockIdx.z / m.gz, bz = blockIdx.z - it * m.gz;")
+        w("  const %s &p = m.p[it];" % P)
+        w("  const int x0 = p.lo0 + (int)(blockIdx.x * blockDim.x * %d);" % px)
+        w("  const int y0 = p.lo1 + (int)(blockIdx.y * blockDim.y) * %d;" % py)
+        w("  const int z0 = p.lo2 + (int)(bz * blockDim.z);")
+        w("  ob2::hfuse_prologue(h, (int)it, x0, min(x0 + (int)blockDim.x * %d, p.hi0), y0,"
+          " min(y0 + (int)blockDim.y * %d, p.hi1), z0, min(z0 + (int)blockDim.z, p.hi2));" %
+          (px, py))
+        w("  __syncthreads();")
+        w("  ob2ub_%s<false>(p, blockIdx.x, blockIdx.y, bz%s);" %
+          (base, ", false" if aw is not None else ""))
+        w("}")
+        w("static int ob2l_%s_u(const void *prm, const unsigned *g, const unsigned *b, void *st) {" %
+          base)
+        w("  %sU<<<dim3(g[0], g[1], g[2]), dim3(b[0], b[1], b[2]), 0, (cudaStream_t)st>>>"
+          "(*(const %s *)prm);" % (K, P))
+        w("  return (int)cudaGetLastError();")
+        w("}")
+        for nm, extra, arg in (("m", "", ""), ("h", ", const ob2_hfuse *h", ", *h")):
+            w("static int ob2%s_%s_u(const void *const *prm, int n, const unsigned *g,"
+              " const unsigned *b%s, void *st) {" % (nm, base, extra))
+            w("  if (n < 1 || n > OB2_MULTI_MAX) return (int)cudaErrorInvalidValue;")
+            w("  %sM m;" % P)
+            w("  for (int k = 0; k < n; k++) m.p[k] = *(const %s *)prm[k];" % P)
+            w("  m.gz = g[2];")
+            w("  %sU%s<<<dim3(g[0], g[1], g[2] * n), dim3(b[0], b[1], b[2]), 0,"
+              " (cudaStream_t)st>>>(m%s);" % (K, nm.upper(), arg))
+            w("  return (int)cudaGetLastError();")
+            w("}")
+
     def red_rows(self, dats) -> int:
         """Most consecutive rows per thread and tile of a reduction kernel:
         4 when its dats read at most 24 bytes per point, so that a thread has
@@ -785,7 +963,7 @@ class Translator:
         if self.rpy:
             return self.rpy
         rd = sum(self.ELEM_BYTES.get(p.base_type, 8) for i, a, p in dats if a.acc != "OPS_WRITE")
-        return 4 if rd <= 24 else 1
+        return 4 if rd <= 32 else 1
 
     def align_dat(self, loop: Loop, kd, dats, reds, py):
         """3D loops without reductions and with one row per thread: the first
@@ -963,8 +1141,8 @@ class Translator:
             elif a.kind == "reduce":
                 w("  %s *r%d; %s *part%d; int first%d;" % (p.base_type, i, p.base_type, i, i))
                 reds.append((i, a, p))
-        if reds:  # tiles along x, y and z; rows per thread of a tile
-            w("  unsigned tx, ty, tz; int rows;")
+        if reds:  # tiles along x, y and z; columns and rows per thread of a tile
+            w("  unsigned tx, ty, tz; int cols, rows;")
         w("};")
         # Point function, in two variants: with __restrict__ dat pointers
         # (the common case: no dat is both written and passed twice, so the
@@ -1045,7 +1223,16 @@ class Translator:
                 not self.light_y_stencil(kd) and self.align_dat(loop, kd, dats, reds, 1) is not None):
             py = 1
         aw = self.align_dat(loop, kd, dats, reds, py)
-        if aw is not None:
+        base = loop.stub[len("ops_par_loop_"):]
+        uni = self.uni_dats(loop, dats)
+        if uni:
+            px, pyu = self.uni_shape(loop, kd, dats, reds)
+            awu = aw if px * pyu == 1 else None
+        if uni and reds:  # the reduction kernel below calls its tile function
+            self.emit_uni(loop, kd, P, base, dats, reds, px, pyu, awu, w)
+        if uni and reds:
+            w("template <bool RESTRICT, bool IDX32, bool UNI = false>")
+        elif aw is not None:
             w("template <bool RESTRICT, bool IDX32, bool ALIGN = true>")
         else:
             w("template <bool RESTRICT, bool IDX32>")
@@ -1080,7 +1267,7 @@ class Translator:
             w("  for (unsigned long long t = blockIdx.x; t < nt; t += gridDim.x) {")
             w("    unsigned bx, by, bz;")
             w("    ob2::tile_of(t, nt, p.tx, p.ty, bx, by, bz);")
-            w("    const int x = p.lo0 + (int)(bx * blockDim.x + threadIdx.x);")
+            w("    const int x = p.lo0 + (int)(bx * blockDim.x * p.cols + threadIdx.x);")
             w("    const int yb = p.lo1 + (int)(by * blockDim.y + threadIdx.y) * p.rows;")
             if hd:  # the 3rd to 5th axes as one folded index
                 w("    const int nz = p.hi2 - p.lo2, nu = p.hi3 - p.lo3, nzu = nz * (p.hi4 - p.lo4) * nu;")
@@ -1091,6 +1278,11 @@ class Translator:
             else:
                 w("    const int z = p.lo2 + (int)(bz * blockDim.z + threadIdx.z);")
                 w("    if (x < p.hi0 && z < p.hi2) {")
+            if uni:
+                w("      if (UNI) {")
+                w("        ob2ue_%s<true>(p, x, yb, z%s);" %
+                  (base, "".join(", red%d" % i for i, a, p in reds)))
+                w("      } else")
             # all PY rows in range: no branch between the calls, so the loads
             # of every row can be issued before the stores of the first, and
             # rows shared by the stencils are loaded once
@@ -1213,6 +1405,8 @@ class Translator:
             w("  %s<false, IDX32%s>(p, blockIdx.x, blockIdx.y, bz);" %
               (BF, ", false" if aw is not None else ""))
             w("}")
+        if uni and not reds:
+            self.emit_uni(loop, kd, P, base, dats, reds, px, pyu, awu, w)
         tb = self.tb_candidate(loop, kd)
         if tb:
             self.emit_tblock(loop, kd, P, K, I, dats, tb, w)
@@ -1253,6 +1447,12 @@ class Translator:
               " (cudaStream_t)st>>>(*(const %s *)prm);" % (K, rs, ix, P))
             w("  return (int)cudaGetLastError();")
             w("}")
+        if uni and reds:
+            w("static int %s_u(const void *prm, const unsigned *g, const unsigned *b, void *st) {" % LN)
+            w("  %s<true, true, true><<<dim3(g[0], g[1], g[2]), dim3(b[0], b[1], b[2]), 0,"
+              " (cudaStream_t)st>>>(*(const %s *)prm);" % (K, P))
+            w("  return (int)cudaGetLastError();")
+            w("}")
         # host stub
         params = ", ".join("ops_arg arg%d" % i for i in range(len(loop.args)))
         ns = re.sub(r"\W", "_", self.app)
@@ -1283,14 +1483,47 @@ class Translator:
               (128 // self.ELEM_BYTES[kd.params[aw].base_type] - 1))
         if not reds and py > 1:
             w("  grd.y = (L.n[1] + blk.y * %d - 1) / (blk.y * %d);" % (py, py))
+        w("  const bool al = ob2_args_alias(args, %d) != 0;" % na)
+        if uni:  # one layout for every dat, no aliases, 32-bit offsets
+            k0 = dats[0][0]
+            cond = []
+            for i, a, pr in dats:
+                c = ["L.view[%d].wx == 1" % i]
+                if nd > 1:
+                    c += ["L.view[%d].wy == L.view[%d].ey" % (i, k0)]
+                    c += ["L.view[%d].ey == L.view[%d].ey" % (i, k0)] if i != k0 else []
+                if nd > 2:
+                    c += ["L.view[%d].wz == L.view[%d].ez" % (i, k0)]
+                    c += ["L.view[%d].ez == L.view[%d].ez" % (i, k0)] if i != k0 else []
+                cond.append(" && ".join(c))
+            # a kernel of several points per thread needs enough of them (1.5
+            # waves of 2048 threads per SM with a stencil: a 5-point sweep of
+            # 1500^2 ran at 0.88 (FP64) and 0.73 (FP32) of the other kernel's
+            # speed, 2048^2 at 1.12; half a wave without: p = r + b p of 1000 x
+            # 777 3.7 against 4.8 us), and rows long enough that the tiles cut
+            # off at their end, taken point by point, are few
+            big = " && L.npoints >= %dLL" % (148 * (3072 if pyu > 1 else 1024) * px * pyu) \
+                if not reds and px * pyu > py else ""
+            big += " && L.n[0] >= %d" % (128 * px) if not reds and px > 1 else ""
+            w("  const bool uni = !al && L.idx32%s%s &&\n    %s;" %
+              (" && blk.x == 32" if px > 1 else "", big, " &&\n    ".join(cond)))
+            if not reds and (px > 1 or pyu != py or (awu is None) != (aw is None)):
+                pad = " + %d" % (128 // self.ELEM_BYTES[kd.params[awu].base_type] - 1) \
+                    if awu is not None else ""
+                w("  if (uni) {")
+                w("    grd.x = (unsigned)((L.n[0]%s + (int)blk.x * %d - 1) / ((int)blk.x * %d));" %
+                  (pad, px, px))
+                w("    grd.y = (L.n[1] + blk.y * %d - 1) / (blk.y * %d);" % (pyu, pyu))
+                w("  }")
         if reds:
-            w("  const bool al = ob2_args_alias(args, %d) != 0;" % na)
-            w("  const void *kern = al ? (L.idx32 ? (const void *)%s<false, true> : (const void *)%s"
+            w("  const void *kern = " + ("uni ? (const void *)%s<true, true, true> : " % K if uni else "") + "al ? (L.idx32 ? (const void *)%s<false, true> : (const void *)%s"
               "<false, false>) : (L.idx32 ? (const void *)%s<true, true> : (const void *)%s<true,"
               " false>);" % (K, K, K, K))
             w("  unsigned tiles[3];")
-            w("  grd = dim3(ob2_red_grid(&L, %d, ob2::resident_ctas(kern, (int)(blk.x * blk.y *"
-              " blk.z)), tiles, &p.rows), 1, 1);" % py)
+            w("  p.cols = %s; p.rows = %s;" % ("uni ? %d : 1" % px if uni else "1",
+                                               "uni ? %d : %d" % (pyu, py) if uni else str(py)))
+            w("  grd = dim3(ob2_red_grid(&L, &p.cols, &p.rows, ob2::resident_ctas(kern, (int)"
+              "(blk.x * blk.y * blk.z)), tiles), 1, 1);")
             w("  p.tx = tiles[0]; p.ty = tiles[1]; p.tz = tiles[2];")
             w("  size_t nblk = (size_t)grd.x * grd.y * grd.z;")
             w("  char *scratch = (char *)L.partials;")
@@ -1326,21 +1559,23 @@ class Translator:
                 w("  p.part%d = (%s *)scratch;"
                   " scratch += ((nblk * (%s) * sizeof(%s) + 255) / 256) * 256;" %
                   (i, p.base_type, a.dim, p.base_type))
-        if not reds:
-            w("  const bool al = ob2_args_alias(args, %d) != 0;" % na)
-        w("  const ob2_launcher fn = al ? (L.idx32 ? %s_f_t : %s_f_f)"
-          " : (L.idx32 ? %s_t_t : %s_t_f);" % (LN, LN, LN, LN))
+        w("  const ob2_launcher fn = %sal ? (L.idx32 ? %s_f_t : %s_f_f)"
+          " : (L.idx32 ? %s_t_t : %s_t_f);" % ("uni ? %s_u : " % LN if uni else "", LN, LN, LN, LN))
         w("  const unsigned g3[3] = {grd.x, grd.y, grd.z}, b3[3] = {blk.x, blk.y, blk.z};")
         if reds:
             w("  const ob2_mlauncher mfn = nullptr;")
         else:
-            w("  const ob2_mlauncher mfn = al ? (L.idx32 ? %s_f_t : %s_f_f)"
-              " : (L.idx32 ? %s_t_t : %s_t_f);" % (MN, MN, MN, MN))
+            w("  const ob2_mlauncher mfn = %sal ? (L.idx32 ? %s_f_t : %s_f_f)"
+              " : (L.idx32 ? %s_t_t : %s_t_f);" %
+              ("uni ? %s_u : " % MN if uni else "", MN, MN, MN, MN))
         if not reds and not hd:
-            w("  L.fuse_id = %d;" % len(self.fuse_items))
+            w("  L.fuse_id = %s%d;" % ("uni ? %d : " % (len(self.fuse_items) + 1) if uni else "",
+                                       len(self.fuse_items)))
             w("  L.ffn = ob2f_launch;")
-            w("  L.hfn = L.idx32 ? %s_t : %s_f;" % (HN, HN))
-            self.fuse_items.append((P, "ob2b_" + loop.stub[len("ops_par_loop_"):]))
+            w("  L.hfn = %sL.idx32 ? %s_t : %s_f;" % ("uni ? %s_u : " % HN if uni else "", HN, HN))
+            self.fuse_items.append((P, "ob2b_" + base + "<false, IDX32>"))
+            if uni:
+                self.fuse_items.append((P, "ob2ub_" + base + "<false>"))
         if tb:
             TN = "ob2t_" + loop.stub[len("ops_par_loop_"):]
             offs = ", ".join(("offsetof(%s, b%d)" % (P, i)) if a.kind == "dat" else "0"
@@ -1352,7 +1587,8 @@ class Translator:
             w("  L.tfn = L.idx32 && !al ? %s : nullptr;" % TN)
             w("  L.tb_off = tb_off;")
             w("  L.tb_role = tb_role;")
-        w("  ob2_launch(&L, fn, mfn, &p, sizeof(p), g3, b3, %d);" % (1 if reds else py))
+        w("  ob2_launch(&L, fn, mfn, &p, sizeof(p), g3, b3, %s);" %
+          ("1" if reds else "uni ? %d : %d" % (pyu, py) if uni else str(py)))
         w("  ob2_loop_end(&L);")
         w("}")
         w("namespace ob2_%s {" % ns)
