@@ -35,6 +35,8 @@ typedef struct ob2_red {
   void *acc;    /* device accumulator of the handle (dim values) */
   int first;    /* 1: this loop initialises the accumulator */
   int op;       /* OPS_INC / OPS_MIN / OPS_MAX */
+  unsigned long long *slots;  /* the handle's pinned slots (ob2::publish) */
+  unsigned long long key;     /* this launch's key */
 } ob2_red;
 
 /* A generated fused launcher (one per application): runs n (<= OB2_FUSE_MAX)

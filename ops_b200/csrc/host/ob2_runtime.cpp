@@ -84,6 +84,9 @@ struct RedX {
   void *acc_d = nullptr;   // device accumulator
   int pending_first = 0;   // next loop initialises the accumulator
   void *host_pinned = nullptr;
+  unsigned long long *slots = nullptr;  // pinned: two words per 8 bytes of the result
+  unsigned long long seq = 0, key = 0;  // launches that fed the handle; the last one's key
+  int dim = 0;                          // ... and components
 };
 
 struct GroupX {
@@ -1887,8 +1890,36 @@ OPS_API ops_reduction ops_decl_reduction_handle(int size, const char *type, cons
   RedX x;
   check(ob2_dev_malloc(&x.acc_d, size > 0 ? size : 8), "ops_decl_reduction_handle");
   check(ob2_host_alloc_pinned(&x.host_pinned, size > 0 ? size : 8), "ops_decl_reduction_handle");
+  const size_t room = (size_t)(size > 0 ? size : 8) * 16;  // components of 1 byte and more
+  check(ob2_host_alloc_pinned((void **)&x.slots, room), "ops_decl_reduction_handle");
+  memset(x.slots, 0, room);
   rt().redx.push_back(x);
   return r;
+}
+
+/* Waits for the result that the handle's last loop publishes (ob2::publish,
+ * ops_b200_kernel.h) and stores it in h->data.  False when it is long in
+ * coming (much work ahead of it, or a launch that failed): the caller then
+ * copies it from the device, which also reports errors. */
+static bool take_result(ops_reduction h, RedX &x) {
+  const int ts = type_bytes(type_code(h->type));
+  if (ts < 1) return false;
+  const int words = (ts + 7) / 8;
+  const double t0 = wall();
+  for (int d = 0; d < x.dim && (d + 1) * ts <= h->size; d++)
+    for (int k = 0; k < words; k++) {
+      const unsigned long long *s = x.slots + 2 * (d * words + k);
+      unsigned long long a, b;
+      for (unsigned n = 1;; n++) {
+        a = __atomic_load_n(s, __ATOMIC_RELAXED);
+        b = __atomic_load_n(s + 1, __ATOMIC_RELAXED);
+        if (b == (a ^ x.key)) break;
+        if (n % 256 == 0 && wall() - t0 > 2e-3) return false;
+      }
+      memcpy(h->data + d * ts + 8 * k, &a, std::min(8, ts - 8 * k));
+    }
+  __atomic_thread_fence(__ATOMIC_ACQUIRE);
+  return true;
 }
 
 /* ops_lib_core.cpp:1143-1149: forces execution, returns, resets the handle */
@@ -1896,9 +1927,11 @@ OPS_API void ops_reduction_result_char(ops_reduction h, int, char *ptr) {
   Runtime &r = rt();
   RedX &x = r.redx[h->index];
   if (!x.pending_first) {
-    check(ob2_dev_d2h_async(x.host_pinned, x.acc_d, h->size), "ops_reduction_result");
-    check(ob2_dev_sync(), "ops_reduction_result");
-    memcpy(h->data, x.host_pinned, h->size);
+    if (!take_result(h, x)) {
+      check(ob2_dev_d2h_async(x.host_pinned, x.acc_d, h->size), "ops_reduction_result");
+      check(ob2_dev_sync(), "ops_reduction_result");
+      memcpy(h->data, x.host_pinned, h->size);
+    }
   } else if (r.dist && h->initialized) {
     // no point of this rank's rows fed the handle: its part is the identity
     const int tc = type_code(h->type);
@@ -2474,6 +2507,10 @@ OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int d
       L->red[i].acc = x.acc_d;
       L->red[i].first = x.pending_first;
       L->red[i].op = a.acc;
+      x.key = (++x.seq) * 0x9e3779b97f4a7c15ULL;  // odd factor: another key for every launch
+      L->red[i].slots = x.slots;
+      L->red[i].key = x.key;
+      x.dim = a.dim;
       x.pending_first = 0;
       nred++;
     }

@@ -1140,6 +1140,7 @@ class Translator:
                 w("  %s g%d[%s];" % (p.base_type, i, self.gbl_extent(a.dim)))
             elif a.kind == "reduce":
                 w("  %s *r%d; %s *part%d; int first%d;" % (p.base_type, i, p.base_type, i, i))
+                w("  unsigned long long *rs%d, rk%d;" % (i, i))
                 reds.append((i, a, p))
         if reds:  # tiles along x, y and z; columns and rows per thread of a tile
             w("  unsigned tx, ty, tz; int cols, rows;")
@@ -1365,7 +1366,8 @@ class Translator:
             w("  if (ob2::last_block(p.counter, &ob2_flag)) {")
             for i, a, p in reds:
                 w("    ob2::final_combine<%s, %s>(%s, p.part%d, p.r%d, p.first%d,"
-                  " (%s *)ob2_sh_raw);" % (p.base_type, a.acc, a.dim, i, i, i, p.base_type))
+                  " (%s *)ob2_sh_raw, p.rs%d, p.rk%d);" %
+                  (p.base_type, a.acc, a.dim, i, i, i, p.base_type, i, i))
             w("    ob2::reset_counter(p.counter);")
             w("  }")
         w("}")
@@ -1556,6 +1558,7 @@ class Translator:
             elif a.kind == "reduce":
                 w("  p.r%d = (%s *)L.red[%d].acc; p.first%d = L.red[%d].first;" %
                   (i, p.base_type, i, i, i))
+                w("  p.rs%d = L.red[%d].slots; p.rk%d = L.red[%d].key;" % (i, i, i, i))
                 w("  p.part%d = (%s *)scratch;"
                   " scratch += ((nblk * (%s) * sizeof(%s) + 255) / 256) * 256;" %
                   (i, p.base_type, a.dim, p.base_type))
