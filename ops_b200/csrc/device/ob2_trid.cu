@@ -104,11 +104,6 @@ __device__ __forceinline__ long long line_base(long long line, long long nlines,
   return (long long)(l - q * (unsigned)o1n) * o1s + (long long)q * o2s;
 }
 
-// asks for the line of *p in L2
-__device__ __forceinline__ void prefetch_l2(const void *p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
 // Unit-stride lines.  One segment (SEG 0, lines of up to W * CL points): a
 // group of W lanes per line.  Several: W = 32, the S warps of a line in one
 // CTA, 8 / S lines per CTA (SEG 1), or one line of 9 to 16 warps (SEG 2).
@@ -121,9 +116,8 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
 // of the whole line in shared memory), 36 us FP32 (84).
 template <typename T, bool INC, int SEG, int CL, int W>
 __global__ void __launch_bounds__(SEG == 2 ? 32 * kMaxSeg : kThreads, SEG == 2 ? 1 : 3) trid_x_kernel(
-    int n, int S, int ahead, long long nlines, int o1n, long long o1s, long long o2s,
-    const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ C, T *__restrict__ D,
-    T *__restrict__ U) {
+    int n, int S, long long nlines, int o1n, long long o1s, long long o2s, const T *__restrict__ A,
+    const T *__restrict__ B, const T *__restrict__ C, T *__restrict__ D, T *__restrict__ U) {
   static_assert(!SEG || W == 32, "a segment is a warp's");
   __shared__ double sm[SEG ? kMaxSeg * (6 + 2 * kMaxSeg) : 1];
   const int lane = threadIdx.x % W;
@@ -135,10 +129,6 @@ __global__ void __launch_bounds__(SEG == 2 ? 32 * kMaxSeg : kThreads, SEG == 2 ?
   const int k0 = (seg * W + lane) * CL;
   const int len = active ? max(0, min(CL, n - k0)) : 0;
   const long long base = active ? line_base(line, nlines, o1n, o1s, o2s) + k0 : 0;
-  if (INC && len > 0) {
-    prefetch_l2(U + base);
-    prefetch_l2(U + base + len - 1);
-  }
   double a[CL], b[CL], c[CL], d[CL];
   if (len == CL) {
     load_chunk<T, CL>(A + base, a);
@@ -162,20 +152,6 @@ __global__ void __launch_bounds__(SEG == 2 ? 32 * kMaxSeg : kThreads, SEG == 2 ?
   for (int i = 0; i < CL; i++)
     if (k0 + i == n - 1) c[i] = 0.0;  // no right neighbour
   chunk_reduce<CL>(a, b, c, d);
-  if (ahead) {  // the lines that this place in the grid takes a wave later
-    const long long line2 = line + (long long)ahead * lpc;
-    if (line2 < nlines && len > 0) {
-      const long long b2 = line_base(line2, nlines, o1n, o1s, o2s) + k0;
-#pragma unroll
-      for (int i = 0; i < CL; i += 32 / (int)sizeof(T))
-        if (i < len) {
-          prefetch_l2(A + b2 + i);
-          prefetch_l2(B + b2 + i);
-          prefetch_l2(C + b2 + i);
-          prefetch_l2(D + b2 + i);
-        }
-    }
-  }
   double xf, xl;
   if (SEG == 0 && sizeof(T) == 8) {
     pair_pcr<W>(a[0], c[0], d[0], a[CL - 1], c[CL - 1], d[CL - 1], lane, xf, xl);
@@ -239,8 +215,8 @@ __global__ void __launch_bounds__(SEG == 2 ? 32 * kMaxSeg : kThreads, SEG == 2 ?
 //   2048x1500   y FP64 89 -> 45 us, _Inc 187 -> 60; FP32 103 -> 38, 224 -> 48
 template <typename T, bool INC, bool IDX32, bool SEG, int CL, int W>
 __global__ void __launch_bounds__(kThreads, 3) trid_s_kernel(
-    int n, int S, int ahead, long long nlines, long long stride, int o1n, long long o1s,
-    long long o2s, const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ C,
+    int n, int S, long long nlines, long long stride, int o1n, long long o1s, long long o2s,
+    const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ C,
     T *__restrict__ D, T *__restrict__ U) {
   constexpr int LPB = kThreads / W, pitch = W + 1, field = LPB * pitch;
   __shared__ double sm[6 * field];
@@ -257,13 +233,6 @@ __global__ void __launch_bounds__(kThreads, 3) trid_s_kernel(
     base = IDX32 ? (long long)((int)base + k0 * (int)stride) : base + (long long)k0 * stride;
   }
   const int len = active ? max(0, min(CL, n - k0)) : 0;
-  // one lane per 32-byte sector of a run, and the last
-  const bool fetches = l % (32 / (int)sizeof(T)) == 0 || l == LPB - 1;
-  if (INC && fetches)  // u is needed late
-#pragma unroll
-    for (int i = 0; i < CL; i++)
-      if (i < len)
-        prefetch_l2(U + (IDX32 ? (long long)((int)base + i * (int)stride) : base + i * stride));
   double a[CL], b[CL], c[CL], d[CL];
   if (sizeof(T) == 8 && len == CL) {  // every load of the chunk in flight at once
 #pragma unroll
@@ -321,21 +290,6 @@ __global__ void __launch_bounds__(kThreads, 3) trid_s_kernel(
 #pragma unroll
     for (int i = 0; i < CL; i++)
       if (i < len) u[i] = U[IDX32 ? (long long)((int)base + i * (int)stride) : base + i * stride];
-  }
-  if (ahead && fetches) {  // the lines that this CTA's place takes a wave later
-    const long long line2 = line + (long long)ahead * LPB;
-    if (line2 < nlines) {
-      const long long b2 = line_base(line2, nlines, o1n, o1s, o2s) + (long long)k0 * stride;
-#pragma unroll
-      for (int i = 0; i < CL; i++)
-        if (i < len) {
-          const long long e = IDX32 ? (long long)((int)b2 + i * (int)stride) : b2 + i * stride;
-          prefetch_l2(A + e);
-          prefetch_l2(B + e);
-          prefetch_l2(C + e);
-          prefetch_l2(D + e);
-        }
-    }
   }
   {
     double *q = sm + l * pitch + p;
@@ -513,13 +467,6 @@ bool offsets_fit32(const Lines &g) {
   return mx < 0x7fffffffLL;
 }
 
-// CTAs of a wave (three per SM)
-int wave_ahead() {
-  int sms = 148;
-  ob2_dev_sm_count(&sms);
-  return getenv("OB2_TRID_AHEAD") ? atoi(getenv("OB2_TRID_AHEAD")) : 3 * sms;
-}
-
 template <typename T, bool INC, int SEG, int CL, int W>
 int launch_x(const Lines &g, int S, const Args &q) {
   const int lpc = SEG ? std::max(1, kThreads / 32 / S) : kThreads / W;
@@ -527,8 +474,8 @@ int launch_x(const Lines &g, int S, const Args &q) {
   const long long grid = (g.nlines + lpc - 1) / lpc;
   if (grid > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   trid_x_kernel<T, INC, SEG, CL, W><<<(unsigned)grid, threads, 0, (cudaStream_t)ob2_dev_stream()>>>(
-      g.n, S, SEG ? 0 : wave_ahead(), g.nlines, g.o1n, g.o1s, g.o2s, (const T *)q.a,
-      (const T *)q.b, (const T *)q.c, (T *)q.d, (T *)q.u);
+      g.n, S, g.nlines, g.o1n, g.o1s, g.o2s, (const T *)q.a, (const T *)q.b, (const T *)q.c,
+      (T *)q.d, (T *)q.u);
   return (int)cudaGetLastError();
 }
 
@@ -572,9 +519,9 @@ int launch_s(const Lines &g, int S, const Args &q) {
       if (e != cudaSuccess) return (int)e;
     }
   }
-  return (int)cudaLaunchKernelEx(&cfg, kern, g.n, S, SEG ? 0 : wave_ahead(), g.nlines, g.stride,
-                                 g.o1n, g.o1s, g.o2s, (const T *)q.a, (const T *)q.b,
-                                 (const T *)q.c, (T *)q.d, (T *)q.u);
+  return (int)cudaLaunchKernelEx(&cfg, kern, g.n, S, g.nlines, g.stride, g.o1n, g.o1s, g.o2s,
+                                 (const T *)q.a, (const T *)q.b, (const T *)q.c, (T *)q.d,
+                                 (T *)q.u);
 }
 
 // CL: the fewest rows per chunk that hold the line (fewer idle lanes and
