@@ -28,6 +28,29 @@ def test_reduction_tiles(args):
     assert_lines_close(result_lines(gout), result_lines(cout), 1e-11)
 
 
+@pytest.mark.parametrize("name,args", [
+    ("poisson_mb", ["-nb=1", "-n=1921", "-sweeps=2", "-check=1"]),
+    ("poisson_mb", ["-nb=1", "-n=2048", "-sweeps=2", "-check=1"]),
+    ("heat_cg", ["-n=1301", "-maxit=2", "-prec=both"])])
+def test_common_layout_tiles(name, args):
+    """Ranges large enough for the kernels of several columns per thread: a
+    5-point sweep (4 columns, 2 rows) and the copies, updates and reductions
+    of a CG, whole tiles and tiles cut off at the right and upper edge.  The
+    sweep's dats equal the oracle's but for the boundary's sin(); the CG's
+    dot products are summed in another order, so its FP64 dats agree to 1e-10
+    of the field's scale and the mixed form's to 1e-5 (a beta that rounds to
+    the other float moves every point by one float ulp)."""
+    _, gd = run_app(name, "b200", args, dump=True)
+    _, cd = run_app(name, "oracle", args, dump=True)
+    diffs = compare(gd, cd, floor_frac=1.0)
+    assert diffs
+    for dat, d in diffs.items():
+        if name == "poisson_mb":
+            assert d <= 1e-12, (dat, d)
+        else:
+            assert d <= (1e-5 if dat in ("x", "r32", "p32", "w32") else 1e-10), (dat, d)
+
+
 LINES = [2, 5, 40, 41, 48, 49, 64, 65, 80, 96, 97, 128, 129, 160, 161, 192, 193, 224, 225, 256,
          257, 511, 1537, 2048, 2049, 4096]
 
