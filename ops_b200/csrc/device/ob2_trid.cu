@@ -233,6 +233,18 @@ __global__ void __launch_bounds__(kThreads, 3) trid_s_kernel(
     base = IDX32 ? (long long)((int)base + k0 * (int)stride) : base + (long long)k0 * stride;
   }
   const int len = active ? max(0, min(CL, n - k0)) : 0;
+  // u is added last: its sectors are asked for in L2 with the loads below, each
+  // by the lane that begins it (and the last lane, which may begin one).
+  // Measured, FP64 _Inc: 333x77x300 y 131 -> 117 us, 193x131x67 z 37.1 -> 33.0,
+  // 256^3 y 215 -> 206.  FP32 gets slower (256^3 y 133 -> 149 us), and the
+  // segments of long lines by 1 to 2 % (2048x1500 y 61.3 -> 62.2 us).
+  if (INC && !SEG && sizeof(T) == 8 && (l % 4 == 0 || l == LPB - 1)) {
+#pragma unroll
+    for (int i = 0; i < CL; i++)
+      if (i < len)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(
+            U + (IDX32 ? (long long)((int)base + i * (int)stride) : base + i * stride)));
+  }
   double a[CL], b[CL], c[CL], d[CL];
   if (sizeof(T) == 8 && len == CL) {  // every load of the chunk in flight at once
 #pragma unroll
