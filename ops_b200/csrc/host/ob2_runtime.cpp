@@ -1904,9 +1904,11 @@ OPS_API ops_reduction ops_decl_reduction_handle(int size, const char *type, cons
 static bool take_result(ops_reduction h, RedX &x) {
   const int ts = type_bytes(type_code(h->type));
   if (ts < 1) return false;
+  // components that the last loop did not feed are only in the accumulator
+  if (x.dim * ts != h->size) return false;
   const int words = (ts + 7) / 8;
   const double t0 = wall();
-  for (int d = 0; d < x.dim && (d + 1) * ts <= h->size; d++)
+  for (int d = 0; d < x.dim; d++)
     for (int k = 0; k < words; k++) {
       const unsigned long long *s = x.slots + 2 * (d * words + k);
       unsigned long long a, b;
