@@ -204,12 +204,12 @@ def request_bytes_moved(r: Request, mode: int) -> float:
     the update pass reads p' and w and updates x (FP64) and r (FP64: 80 B
     per point; mixed, with FP32 r, w, p and the FP64 x: 48 B); per residual
     replacement the FP64 residual pass reads x and b and writes r (24 B).
-    ADI: 72 B per point per step (preproc reads u and writes du, the x and y
-    solves read and write du, the z solve reads du and updates u)."""
+    ADI: 56 B per point per step (the x solve reads u and writes du, the y
+    solve reads and writes du, the z solve reads du and updates u)."""
     if r.kind in (POISSON2D, HEAT2D):
         per, outer = (48.0, 24.0) if mode == MIXED else (80.0, 24.0)
         return r.n * r.n * (per * r.iterations + outer * (r.outer + 1))
-    return r.n ** 3 * 72.0 * r.steps
+    return r.n ** 3 * 56.0 * r.steps
 
 
 def serve(engine: Engine, stream: List[Request], budget_bytes: int, iters: int = 16,
@@ -288,7 +288,7 @@ def main(argv=None) -> int:
                     help="arrivals per second (0: all requests at t = 0)")
     ap.add_argument("--mode", default="both", choices=["mixed", "fp64", "both"])
     ap.add_argument("--budget-gb", type=float, default=160.0)
-    ap.add_argument("--iters", type=int, default=16, help="engine iterations per graph replay")
+    ap.add_argument("--iters", type=int, default=16, help="engine iterations per launch")
     ap.add_argument("--tile-y", type=int, default=32)
     ap.add_argument("--inner-tol", type=float, default=1e-2,
                     help="residual drop between FP64 residual replacements")
