@@ -1889,10 +1889,11 @@ OPS_API ops_reduction ops_decl_reduction_handle(int size, const char *type, cons
   rt().reds.push_back(r);
   RedX x;
   check(ob2_dev_malloc(&x.acc_d, size > 0 ? size : 8), "ops_decl_reduction_handle");
-  check(ob2_host_alloc_pinned(&x.host_pinned, size > 0 ? size : 8), "ops_decl_reduction_handle");
-  const size_t room = (size_t)(size > 0 ? size : 8) * 16;  // components of 1 byte and more
-  check(ob2_host_alloc_pinned((void **)&x.slots, room), "ops_decl_reduction_handle");
+  // one pinned buffer: the slots, then room for a copy of the accumulator
+  const size_t bytes = size > 0 ? size : 8, room = bytes * 16;  // components of 1 byte and more
+  check(ob2_host_alloc_pinned((void **)&x.slots, room + bytes), "ops_decl_reduction_handle");
   memset(x.slots, 0, room);
+  x.host_pinned = (char *)x.slots + room;
   rt().redx.push_back(x);
   return r;
 }
