@@ -126,7 +126,11 @@ __device__ __forceinline__ double hash_uniform(int seed, int i, int j, int k) {
 // the neighbours, and recomputing r + beta p there avoids a separate pass.
 
 constexpr int CTA_Y = 8;
-constexpr int NPART = 2;  // partial sums per tile: (p', w) and (r, r)
+// partial sums per tile: (p', w), (r, r) and, at a heat request's new time
+// step, ||b||^2.  The last has a column of its own: it is read after the same
+// barrier as (r, r), and a CTA that is done with it goes on to write (p', w)
+// while the others still read.
+constexpr int NPART = 3;
 
 // two adjacent elements of type T
 template <typename T> struct V2;
@@ -352,9 +356,7 @@ __device__ __forceinline__ void xr_tile(const Pois &q, int t, int g, double (*sh
   group_sum<2>(v, sh, g);
   if (threadIdx.x % GT == 0) {
     q.part[NPART * t + 1] = v[0];
-    // column 0 is free in phase 0 (pw_tile did not run): ||b||^2 of a new
-    // heat time step
-    if (ph == 0 && q.newstep) q.part[NPART * t] = v[1];
+    if (ph == 0 && q.newstep) q.part[NPART * t + 2] = v[1];
   }
 }
 
@@ -383,7 +385,7 @@ __device__ __forceinline__ void advance(Pois &q, double (*sh)[CTA_Y], int grp) {
   const int ph = q.phase;
   const bool newstep = ph == 0 && q.newstep;  // uniform over the group
   const double g = request_sum(q, 1, sh, grp);
-  const double bb = newstep ? request_sum(q, 0, sh, grp) : 0.0;
+  const double bb = newstep ? request_sum(q, 2, sh, grp) : 0.0;
   if (threadIdx.x % GT != 0) return;
   if (ph == 0 || ph == 3) {  // g = (b - A x, b - A x) in FP64
     if (newstep) {  // heat: relative to the step's right-hand side
@@ -471,9 +473,10 @@ __device__ __forceinline__ void xr_any(const Pois &q, int t, int g, double (*sh)
 // grid barriers per iteration in place of four kernel boundaries and two
 // one-CTA-per-request scalar kernels.
 //
-// Between the barriers a request's partial sums of column 0 (column 1) are
-// written by pw_tile (xr_tile) before, and read by form_alpha (advance)
-// after the barrier; the next write follows the next barrier.
+// A request's partial sums of column 0 (columns 1 and 2) are written by
+// pw_tile (xr_tile) before a barrier and read by form_alpha (advance) after
+// it; between the reads and the next write of a column lies the iteration's
+// other barrier.
 template <typename TI>
 __global__ void __launch_bounds__(GT * pois_groups<TI>(), 1) pois_iterate(
     const Work *__restrict__ W, Req *R, int iters, unsigned *bar, unsigned base) {

@@ -118,6 +118,36 @@ def test_heat_requests(mode):
         eng.close()
 
 
+@pytest.mark.parametrize("mode", [serving.FP64, serving.MIXED])
+def test_heat_steps_same_alone_and_in_mix(mode):
+    """Heat requests of several time steps, one of them over more tiles than
+    there are CTAs, among many small requests (a CTA then advances several
+    requests in turn): the norm that each step's residuals are relative to is
+    read by every CTA of the request while the quickest of them start the next
+    pass.  Bit-identical alone and in the mix, three times over."""
+    cases = [(serving.HEAT2D, 700, 3, 4), (serving.HEAT2D, 130, 4, 6), (serving.HEAT2D, 40, 5, 9)]
+    eng = serving.Engine(mode)
+    try:
+        alone = {}
+        for kind, n, seed, steps in cases:
+            rid = eng.submit(kind, n, seed, steps)
+            res = finish_all(eng)[rid]
+            alone[n] = (eng.fetch(rid, n * n), res.iterations, res.outer)
+            eng.release(rid)
+        for _ in range(3):
+            small = [eng.submit(serving.POISSON2D, 16 + 3 * k, k) for k in range(40)]
+            ids = {eng.submit(*c): c[1] for c in cases}
+            small += [eng.submit(serving.HEAT2D, 20 + k, k, 3) for k in range(20)]
+            res = finish_all(eng)
+            for rid, n in ids.items():
+                assert (res[rid].iterations, res[rid].outer) == alone[n][1:], n
+                assert np.array_equal(eng.fetch(rid, n * n), alone[n][0]), n
+            for rid in small + list(ids):
+                eng.release(rid)
+    finally:
+        eng.close()
+
+
 @pytest.mark.parametrize("n,steps", [(24, 3), (41, 2), (70, 1)])
 def test_adi_matches_oracle(n, steps):
     eng = serving.Engine(serving.MIXED)
