@@ -847,8 +847,11 @@ OB2_API int ob2s_create(ob2s_engine **out, int mode, double tol, double inner_to
       (err = cudaMalloc(&e->R_d, sizeof(Req) * (MAXA + 1))) != cudaSuccess ||
       (err = cudaMallocHost(&e->R, sizeof(Req) * (MAXA + 1))) != cudaSuccess ||
       (err = cudaMalloc(&e->W_d, sizeof(Work))) != cudaSuccess ||
-      (err = cudaMemset(e->R_d, 0, sizeof(Req) * (MAXA + 1))) != cudaSuccess ||
-      (err = cudaMemset(e->W_d, 0, sizeof(Work))) != cudaSuccess ||
+      // cleared on the engine's stream, which every later access is ordered
+      // behind (it does not wait for the default stream, whose work may be
+      // long in coming)
+      (err = cudaMemsetAsync(e->R_d, 0, sizeof(Req) * (MAXA + 1), e->st)) != cudaSuccess ||
+      (err = cudaMemsetAsync(e->W_d, 0, sizeof(Work), e->st)) != cudaSuccess ||
       (err = cudaFuncSetAttribute(mode == OB2S_MIXED ? (const void *)pois_iterate<float>
                                                      : (const void *)pois_iterate<double>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,

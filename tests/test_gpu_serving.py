@@ -77,6 +77,29 @@ def test_poisson_meets_tolerance(mode):
         eng.close()
 
 
+def test_engine_made_beside_work_on_the_default_stream():
+    """The engine's slots and grid-barrier words are cleared in the order of
+    its own stream: an engine made and run while the default stream is busy
+    for half a second solves as it does on an idle device."""
+    import torch
+    sol = []
+    for busy in (False, True):
+        torch.cuda.synchronize()
+        if busy:
+            torch.cuda._sleep(1_000_000_000)  # cycles, on the default stream
+        eng = serving.Engine(serving.FP64)
+        try:
+            rid = eng.submit(serving.POISSON2D, 220, 9)
+            res = finish_all(eng)[rid]
+            assert res.done == 1
+            sol.append((eng.fetch(rid, 220 * 220), res.iterations))
+            eng.release(rid)
+        finally:
+            eng.close()
+    torch.cuda.synchronize()
+    assert sol[0][1] == sol[1][1] and np.array_equal(sol[0][0], sol[1][0])
+
+
 def test_mixed_matches_fp64_solution():
     sol = {}
     for mode in (serving.FP64, serving.MIXED):
