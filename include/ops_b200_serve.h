@@ -88,8 +88,13 @@ OB2_API size_t ob2s_request_bytes(int mode, int kind, int n);
  * set at the next ob2s_run.  steps: ADI or heat time steps (ignored for
  * Poisson). */
 OB2_API int ob2s_submit(ob2s_engine *e, int kind, int n, int seed, int steps, int *id);
-/* Runs `iters` engine iterations and waits for them; *n_done: requests finished since
- * the last call, their ids in ids[0..cap). */
+/* Runs `iters` engine iterations and waits for them; *n_done: requests finished
+ * since the last call, their ids in ids[0..cap).
+ * The grid barriers' waits are bounded (seconds; OB2S_BARRIER_POLLS polls in
+ * the environment of ob2s_create).  A run in which one gave up returns
+ * cudaErrorLaunchTimeout and ends the engine: every later ob2s_run and
+ * ob2s_submit returns the same error at once; requests that had finished can
+ * still be asked for, fetched and released. */
 OB2_API int ob2s_run(ob2s_engine *e, int iters, int *ids, int cap, int *n_done);
 OB2_API int ob2s_active(ob2s_engine *e);
 OB2_API int ob2s_result_of(ob2s_engine *e, int id, ob2s_result *res);

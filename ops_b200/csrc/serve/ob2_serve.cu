@@ -427,21 +427,26 @@ __device__ __forceinline__ void advance(Pois &q, double (*sh)[CTA_Y], int grp) {
 
 // Grid barrier of a cooperative launch.  bar[0] counts arrivals for the
 // engine's life (`target` is its value, modulo 2^32, when all CTAs of this
-// barrier have arrived); the wait is bounded, and a CTA that gives up sets
-// bar[1], which makes every other one give up.  False in every thread when
-// the barrier failed.
-constexpr unsigned kSpin = 1u << 22;  // polls of some 0.5 us: seconds
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int *ok) {
+// barrier have arrived; a CTA still here sees less than a grid's arrivals
+// more).  The wait is bounded: the first CTA that gives up sets bar[1] and
+// adds kGaveUp to the count, which every other one finds in the word that it
+// polls anyway and gives up too.  False in every thread when the barrier
+// failed.
+constexpr unsigned kPolls = 1u << 22;  // of some 0.5 us: seconds
+constexpr unsigned kGaveUp = 1u << 30;
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, unsigned polls,
+                                             int *ok) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned seen, k = 0;
+    int over = -1;  // arrivals beyond the target
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    do {
+    for (unsigned k = 0; k < polls && over < 0; k++) {
+      unsigned seen;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-    } while ((int)(seen - target) < 0 && ++k < kSpin);
-    bool good = (int)(seen - target) >= 0;
-    if (!good) atomicExch(bar + 1, 1u);
-    *ok = good;
+      over = (int)(seen - target);
+    }
+    if (over < 0 && atomicExch(bar + 1, 1u) == 0) atomicAdd(bar, kGaveUp);
+    *ok = over >= 0 && over < (int)(kGaveUp / 2);
   }
   __syncthreads();
   return *ok != 0;
@@ -479,7 +484,7 @@ __device__ __forceinline__ void xr_any(const Pois &q, int t, int g, double (*sh)
 // other barrier.
 template <typename TI>
 __global__ void __launch_bounds__(GT * pois_groups<TI>(), 1) pois_iterate(
-    const Work *__restrict__ W, Req *R, int iters, unsigned *bar, unsigned base) {
+    const Work *__restrict__ W, Req *R, int iters, unsigned *bar, unsigned base, unsigned polls) {
   constexpr int NG = pois_groups<TI>();
   __shared__ double shs[NG][2][CTA_Y];
   __shared__ int ok;
@@ -509,7 +514,7 @@ __global__ void __launch_bounds__(GT * pois_groups<TI>(), 1) pois_iterate(
       if (!q.done && q.phase == 2) pw_any<TI>(q, (int)(u - W->pois_pref[k]), g, sh);
     }
     base += gridDim.x;
-    if (!grid_barrier(bar, base, &ok)) return;
+    if (!grid_barrier(bar, base, polls, &ok)) return;
     for (int k = g; k < nk; k += NG) form_alpha(qs[k], sh, g);
     __syncthreads();
     for (long long u = t0 + g; u < t1; u += NG) {
@@ -518,7 +523,7 @@ __global__ void __launch_bounds__(GT * pois_groups<TI>(), 1) pois_iterate(
       if (!q.done) xr_any<TI>(q, (int)(u - W->pois_pref[k]), g, sh);
     }
     base += gridDim.x;
-    if (!grid_barrier(bar, base, &ok)) return;
+    if (!grid_barrier(bar, base, polls, &ok)) return;
     for (int k = g; k < nk; k += NG) advance(qs[k], sh, g);
     __syncthreads();
   }
@@ -779,6 +784,8 @@ struct ob2s_engine {
   bool work_dirty;
   unsigned *bar_d;     // grid barrier of pois_iterate (arrivals, failure), in R_d's last slot
   unsigned bar_base;   // arrivals before the next launch
+  unsigned polls;      // of a grid barrier before it gives up
+  int failed;          // error of the run whose grid barrier gave up
   long long launches;
   // the requests' memory: a pool of the engine's own that keeps freed
   // memory mapped (a request admitted after another retired reuses its
@@ -804,7 +811,7 @@ static size_t pois_smem() { return sizeof(Pois) * MAXA; }
 
 // `iters` iterations of the Poisson and heat requests
 static cudaError_t launch_pois(ob2s_engine *e, int iters) {
-  void *args[] = {&e->W_d, &e->R_d, &iters, &e->bar_d, &e->bar_base};
+  void *args[] = {&e->W_d, &e->R_d, &iters, &e->bar_d, &e->bar_base, &e->polls};
   const bool mixed = e->mode == OB2S_MIXED;
   const void *f = mixed ? (const void *)pois_iterate<float> : (const void *)pois_iterate<double>;
   const int threads = GT * (mixed ? pois_groups<float>() : pois_groups<double>());
@@ -861,6 +868,9 @@ OB2_API int ob2s_create(ob2s_engine **out, int mode, double tol, double inner_to
   }
   e->bar_d = (unsigned *)(e->R_d + MAXA);
   e->bar_base = 0;
+  e->polls = kPolls;
+  if (const char *v = getenv("OB2S_BARRIER_POLLS")) e->polls = (unsigned)strtoul(v, nullptr, 10);
+  e->failed = 0;
   {
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
@@ -933,6 +943,7 @@ OB2_API int ob2s_submit(ob2s_engine *e, int kind, int n, int seed, int steps, in
   if (grid2d ? (n < 1 || n > 32768 || (kind == OB2S_HEAT2D && steps < 1))
              : (kind != OB2S_ADI3D || n < 3 || n > ADI_MAX_N || steps < 1))
     return OB2S_ERR_BADARG;
+  if (e->failed) return e->failed;
   int slot = -1;
   for (int k = 0; k < MAXA; k++)
     if (!e->used[k]) {
@@ -1049,6 +1060,7 @@ static int upload_work(ob2s_engine *e) {
 OB2_API int ob2s_run(ob2s_engine *e, int iters, int *ids, int cap, int *n_done) {
   if (iters < 1) return OB2S_ERR_BADARG;
   *n_done = 0;
+  if (e->failed) return e->failed;
   int err;
   if (e->work_dirty && (err = upload_work(e))) return err;
   bool pois = false;
@@ -1072,8 +1084,9 @@ OB2_API int ob2s_run(ob2s_engine *e, int iters, int *ids, int cap, int *n_done) 
                                    e->st);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
   if (ce != cudaSuccess) return rc(ce);
-  if (((const unsigned *)(e->R + MAXA))[1])  // a grid barrier gave up
-    return (int)cudaErrorLaunchTimeout;
+  // a grid barrier gave up: the CTAs stopped in different passes, so the
+  // requests' arrays do not belong together and the barrier's count is off
+  if (((const unsigned *)(e->R + MAXA))[1]) return e->failed = (int)cudaErrorLaunchTimeout;
   for (int k = 0; k < MAXA; k++) {
     if (!e->used[k] || !e->R[k].done) continue;
     if (e->active[k]) {

@@ -100,6 +100,43 @@ def test_engine_made_beside_work_on_the_default_stream():
     assert sol[0][1] == sol[1][1] and np.array_equal(sol[0][0], sol[1][0])
 
 
+def test_barrier_that_gives_up_ends_the_engine(monkeypatch):
+    """A grid barrier without a single poll gives up in every CTA (as one
+    whose wait runs out does): the run returns an error, and so does every
+    later run or submission, at once; a request that had finished can still be
+    fetched, and the device serves another engine."""
+    import time
+    monkeypatch.setenv("OB2S_BARRIER_POLLS", "0")
+    eng = serving.Engine(serving.FP64)
+    try:
+        adi = eng.submit(serving.ADI3D, 24, 77, 3)  # no grid barrier in its steps
+        finish_all(eng)
+        cg = eng.submit(serving.POISSON2D, 700, 1)
+        for _ in range(2):
+            t = time.perf_counter()
+            with pytest.raises(RuntimeError, match="ob2s_run failed"):
+                eng.run(100000)
+            assert time.perf_counter() - t < 1.0
+        with pytest.raises(RuntimeError, match="ob2s_submit failed"):
+            eng.submit(serving.ADI3D, 24, 77, 3)
+        assert eng.result(cg).done == 0
+        u = eng.fetch(adi, 24 ** 3).reshape(24, 24, 24)
+        ref = so.adi_steps(24, 77, 3)
+        assert np.max(np.abs(u - ref)) <= 1e-13 * np.max(np.abs(ref))
+        eng.release(adi)
+        eng.release(cg)
+    finally:
+        eng.close()
+    monkeypatch.delenv("OB2S_BARRIER_POLLS")
+    eng = serving.Engine(serving.FP64)
+    try:
+        rid = eng.submit(serving.POISSON2D, 90, 2)
+        finish_all(eng)
+        assert so.relative_residual(eng.fetch(rid, 90 * 90).reshape(90, 90), 2) <= 1.05e-8
+    finally:
+        eng.close()
+
+
 def test_mixed_matches_fp64_solution():
     sol = {}
     for mode in (serving.FP64, serving.MIXED):
