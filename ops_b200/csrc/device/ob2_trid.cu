@@ -221,6 +221,9 @@ __global__ void __launch_bounds__(kThreads, 3) trid_s_kernel(
   constexpr int LPB = kThreads / W, pitch = W + 1, field = LPB * pitch;
   __shared__ double sm[6 * field];
   extern __shared__ double ends[];  // SEG: [line][segment][6], then [line][segment][2]
+  // a CTA's shared memory may be written by the others once it runs: all say
+  // so here and wait for one another before the first such store below
+  if (SEG) cg::this_cluster().barrier_arrive();
   const int tid = threadIdx.x;
   const int p = tid / LPB, l = tid % LPB;
   const int seg = SEG ? (int)(blockIdx.x % (unsigned)S) : 0;
@@ -326,6 +329,7 @@ __global__ void __launch_bounds__(kThreads, 3) trid_s_kernel(
         __syncthreads();            // every group has read its chunk ends
         put_ends<W>(a0, c0, d0, gA, gC, gD, lane, mine);
         __syncwarp();
+        cl.barrier_wait();  // every CTA of the cluster runs
         for (int k = lane; k < 6 * S; k += W) {
           const int r = k / 6, v = k - 6 * r;
           cl.map_shared_rank(ends, r)[(w * S + seg) * 6 + v] = mine[v];

@@ -70,6 +70,17 @@ def test_trid_line_lengths(typ, solvedim, n):
         test_trid_batch(typ, solvedim, inc, tuple(shape))
 
 
+@pytest.mark.parametrize("typ", ["double", "float"])
+@pytest.mark.parametrize("segments", range(2, 17))
+def test_trid_segments(typ, segments):
+    """Strided lines of 2 to 16 segments (the CTAs of a cluster, which write
+    into each other's shared memory), the last segment partly empty and the
+    last cluster with fewer lines than it holds, three solves in a row."""
+    from tests.test_gpu_cabi import test_trid_batch
+    for inc in (False, True, False):
+        test_trid_batch(typ, 1, inc, (13, 256 * segments - 37, 1))
+
+
 def test_trid_too_long_is_refused():
     """Lines of more than 4096 points: an error, nothing written."""
     import ctypes as C
