@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(SEG == 2 ? 32 * kMaxSeg : kThreads, SEG == 2 ?
 //   193x131x67  z FP64 42 -> 25 us, _Inc 74 -> 37; FP32 68 -> 16, 103 -> 19
 //   2048x1500   y FP64 89 -> 45 us, _Inc 187 -> 60; FP32 103 -> 38, 224 -> 48
 template <typename T, bool INC, bool IDX32, bool SEG, int CL, int W>
-__global__ void __launch_bounds__(kThreads, 3) trid_s_kernel(
+__global__ void __launch_bounds__(kThreads, CL > 8 ? 1 : 3) trid_s_kernel(
     int n, int S, long long nlines, long long stride, int o1n, long long o1s, long long o2s,
     const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ C,
     T *__restrict__ D, T *__restrict__ U) {
@@ -512,6 +512,29 @@ int solve_x(const Lines &g, const Args &q) {
   return few ? launch_x<T, INC, 2, 6, 32>(g, S, q) : launch_x<T, INC, 2, 8, 32>(g, S, q);
 }
 
+// CTAs of a cluster: 16 (more than the portable 8 must be asked for, and a
+// device that is partitioned may not have them), OB2_TRID_CLUSTER for fewer
+int cluster_limit() {
+  static const int v = [] {
+    const char *e = getenv("OB2_TRID_CLUSTER");
+    return e ? std::max(8, std::min(kMaxSeg, atoi(e))) : kMaxSeg;
+  }();
+  return v;
+}
+
+// whether clusters of more than 8 CTAs of the kernel can run here
+template <typename K>
+bool wide_clusters(K kern, const cudaLaunchConfig_t &cfg) {
+  int n = 0;
+  if ((int)cfg.attrs[0].val.clusterDim.x <= cluster_limit() &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+          cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
+    return true;
+  (void)cudaGetLastError();
+  return false;
+}
+
 template <typename T, bool INC, bool IDX32, bool SEG, int CL, int W>
 int launch_s(const Lines &g, int S, const Args &q) {
   constexpr int LPB = kThreads / W;
@@ -530,10 +553,10 @@ int launch_s(const Lines &g, int S, const Args &q) {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (S > 8) {  // more CTAs than the portable cluster size
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return (int)e;
-    }
+    // otherwise segments of twice the rows, 8 of them at most
+    if constexpr (CL <= 8)
+      if (S > 8 && !wide_clusters(kern, cfg))
+        return launch_s<T, INC, IDX32, true, 16, W>(g, (g.n + 16 * W - 1) / (16 * W), q);
   }
   return (int)cudaLaunchKernelEx(&cfg, kern, g.n, S, g.nlines, g.stride, g.o1n, g.o1s, g.o2s,
                                  (const T *)q.a, (const T *)q.b, (const T *)q.c, (T *)q.d,

@@ -205,6 +205,22 @@ def test_trid_strided_kernels(mode, typ):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("typ", ["double", "float"])
+def test_trid_portable_clusters(typ):
+    """OB2_TRID_CLUSTER=8: lines of 2049 to 4096 points in segments of 512
+    points, as on a device without clusters of 16 CTAs (a child process,
+    since the limit is read once per process)."""
+    import subprocess
+    import sys
+    calls = "; ".join("t.test_trid_batch(%r, 1, %r, (9, %d, 1))" % (typ, inc, n)
+                      for n in (2048, 2049, 2561, 4095, 4096) for inc in (False, True))
+    code = ("import sys; sys.path.insert(0, %r); import tests.test_gpu_cabi as t; %s" %
+            (os.path.dirname(os.path.dirname(os.path.abspath(__file__))), calls))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                       env=dict(os.environ, OB2_TRID_CLUSTER="8"), timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_device_memspace_slab_set_and_fetch():
     """The external data access API with device buffers (OPS_DEVICE), as the
     reference's access app uses it (apps/c/access/fetch_data.cu): a 2 x 2 slab
