@@ -209,10 +209,11 @@ def test_trid_strided_kernels(mode, typ):
 def test_trid_portable_clusters(typ):
     """OB2_TRID_CLUSTER=8: lines of 2049 to 4096 points in segments of 512
     points, as on a device without clusters of 16 CTAs (a child process,
-    since the limit is read once per process)."""
+    since the limit is read once per process; test_trid_batch solves a range
+    of two points less than the shape has along y)."""
     import subprocess
     import sys
-    calls = "; ".join("t.test_trid_batch(%r, 1, %r, (9, %d, 1))" % (typ, inc, n)
+    calls = "; ".join("t.test_trid_batch(%r, 1, %r, (7, %d, 2))" % (typ, inc, n + 2)
                       for n in (2048, 2049, 2561, 4095, 4096) for inc in (False, True))
     code = ("import sys; sys.path.insert(0, %r); import tests.test_gpu_cabi as t; %s" %
             (os.path.dirname(os.path.dirname(os.path.abspath(__file__))), calls))

@@ -78,7 +78,7 @@ def test_trid_segments(typ, segments):
     last cluster with fewer lines than it holds, three solves in a row."""
     from tests.test_gpu_cabi import test_trid_batch
     for inc in (False, True, False):
-        test_trid_batch(typ, 1, inc, (13, 256 * segments - 37, 1))
+        test_trid_batch(typ, 1, inc, (7, 256 * segments - 35, 2))
 
 
 def test_trid_too_long_is_refused():
