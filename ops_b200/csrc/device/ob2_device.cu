@@ -251,8 +251,9 @@ OB2_API int ob2_halo_run_noalloc(const ob2_halo_task *tasks_host, int ntasks) {
 // per lane in flight and one division per row; a 187 x 180 x 139 box of 3
 // FP64 components (112 MB each way) takes 39 us against 64 us for one
 // element per thread with two 64-bit divisions and a component loop.
-// Components of a SoA dat lie apart: each is a box of its own (STR) whose
-// buffer elements are nc apart.
+// Components of a SoA dat lie apart: each, and each unit of a wider element,
+// is a box of its own whose buffer elements are nc apart (STR: box first +
+// blockIdx.y of nc * units).
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -263,7 +264,10 @@ struct BoxRows {
   long long len, bstep;         // units per row, buffer units per row
   long long rows;               // c1 * c2
   int c1, npiece, lr;           // rows per plane, pieces per row, log2 lanes
-  int dx, bx;                   // STR: units from one to the next in the dat and the buffer
+  int dx, bx;                   // STR: units from one to the next in the dat (those of an
+                                // element) and the buffer (those of a point)
+  long long comp;               // STR: units from one component to the next in the dat
+  unsigned first;               // STR: box of blockIdx.y 0
   int dir;                      // 0 dat -> buffer, 1 buffer -> dat
 };
 
@@ -271,6 +275,11 @@ template <typename U, bool STR>
 __global__ void __launch_bounds__(256) box_copy_kernel(U *__restrict__ dat, U *__restrict__ buf,
                                                        const BoxRows g) {
   const int lane = threadIdx.x & ((1 << g.lr) - 1), ln = 1 << g.lr;
+  if (STR) {
+    const unsigned k = g.first + blockIdx.y;
+    dat += k / g.dx * g.comp + k % g.dx;
+    buf += k;
+  }
   const long long items = g.rows * g.npiece;
   const long long step = (long long)gridDim.x * (blockDim.x >> g.lr);
   for (long long it = (long long)blockIdx.x * (blockDim.x >> g.lr) + (threadIdx.x >> g.lr);
@@ -321,7 +330,11 @@ int launch_box(char *dat, char *buf, BoxRows g, bool apart) {
   const long long need = (g.rows * g.npiece + per - 1) / per;
   const unsigned blocks = (unsigned)std::min(need, 32LL * g_sms);
   if (apart)
-    box_copy_kernel<U, true><<<blocks, 256, 0, g_stream>>>((U *)dat, (U *)buf, g);
+    for (int k = 0; k < g.bx; k += 65535) {
+      g.first = k;
+      box_copy_kernel<U, true><<<dim3(blocks, std::min(g.bx - k, 65535)), 256, 0, g_stream>>>(
+          (U *)dat, (U *)buf, g);
+    }
   else
     box_copy_kernel<U, false><<<blocks, 256, 0, g_stream>>>((U *)dat, (U *)buf, g);
   return rc(cudaGetLastError());
@@ -352,17 +365,11 @@ OB2_API int ob2_box_copy(char *dat, int ts, int nc, int soa, const int *size3, c
   g.len = apart ? count3[0] : count3[0] * m;
   g.dx = apart ? w : 1;
   g.bx = apart ? nc * w : 1;
-  int e = 0;
-  for (int c = 0; c < (apart ? nc : 1); c++)
-    for (int k = 0; k < (apart ? w : 1) && !e; k++) {
-      char *d = dat + (apart ? (c * sy * size3[2] * w + k) * u : 0);
-      char *b = buf + (apart ? ((long long)c * w + k) * u : 0);
-      e = u == 8   ? launch_box<unsigned long long>(d, b, g, apart)
-          : u == 4 ? launch_box<unsigned int>(d, b, g, apart)
-          : u == 2 ? launch_box<unsigned short>(d, b, g, apart)
-                   : launch_box<unsigned char>(d, b, g, apart);
-    }
-  return e;
+  g.comp = sy * size3[2] * w;
+  return u == 8   ? launch_box<unsigned long long>(dat, buf, g, apart)
+         : u == 4 ? launch_box<unsigned int>(dat, buf, g, apart)
+         : u == 2 ? launch_box<unsigned short>(dat, buf, g, apart)
+                  : launch_box<unsigned char>(dat, buf, g, apart);
 }
 
 // ---------------------------------------------------------------------------

@@ -146,6 +146,37 @@ def test_slab_fetch_and_set(soa, typ, dim):
         L.ops_set_soa(0)
 
 
+def test_slab_of_soa_components_is_one_launch():
+    """All components of a SoA dat, and both halves of a complex element, go
+    in one launch."""
+    import ctypes as C
+
+    import numpy as np
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    from tests import cabi
+    L = cabi.lib()
+    vp, ip = C.c_void_p, C.POINTER(C.c_int)
+    L.ops_dat_fetch_data_slab_memspace.argtypes = [vp, C.c_int, vp, ip, C.c_int]
+    n = [40, 9, 8]
+    L.ops_set_soa(1)
+    try:
+        h = L.ops_decl_dat_char(L.ops_decl_block(3, b"one"), 5, cabi.ivec(n), cabi.ivec([0] * 3),
+                                cabi.ivec([-1] * 3), cabi.ivec([1] * 3), cabi.ivec([1] * 3), None,
+                                16, b"complexd", b"one")
+        out = np.empty((4, 4, 30, 5 * 16), np.uint8)
+        torch.zeros(1, device="cuda")
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            L.ops_dat_fetch_data_slab_memspace(h, 0, out.ctypes.data,
+                                               cabi.ivec([3, 33, 2, 6, 1, 5]), 1)
+            torch.cuda.synchronize()
+    finally:
+        L.ops_set_soa(0)
+    copies = [e for e in prof.events() if "box_copy" in e.name]
+    assert len(copies) == 1, [e.name for e in prof.events()]
+
+
 def test_slab_of_long_rows():
     """Rows of more than one piece (1024 units of 8 bytes), 1D and 2D."""
     import ctypes as C
