@@ -244,16 +244,15 @@ OB2_API int ob2_halo_run_noalloc(const ob2_halo_task *tasks_host, int ntasks) {
 // Box copy between a dat (storage coordinates start3/count3) and a dense AoS
 // buffer, for fetch/set data and slabs (ops_util.cpp:353-500 semantics).
 //
-// Bound by HBM: one read and one write per element.  An AoS box is c1 * c2
-// rows of c0 * nc elements that are contiguous on both sides, so a group of
+// Bound by HBM: one read and one write per element.  A row of the box is
+// c0 * nc elements, contiguous in the buffer and in an AoS dat, so a group of
 // LR lanes (the smallest power of two that covers a row, at most a warp)
 // copies a row, or a piece of kPiece units of a long one, with four accesses
 // per lane in flight and one division per row; a 187 x 180 x 139 box of 3
 // FP64 components (112 MB each way) takes 39 us against 64 us for one
 // element per thread with two 64-bit divisions and a component loop.
-// Components of a SoA dat lie apart: each, and each unit of a wider element,
-// is a box of its own whose buffer elements are nc apart (STR: box first +
-// blockIdx.y of nc * units).
+// Components of a SoA dat lie apart (SOA): the lanes take the units of the
+// buffer's row in turn, each from its component's own row in the dat.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -264,24 +263,18 @@ struct BoxRows {
   long long len, bstep;         // units per row, buffer units per row
   long long rows;               // c1 * c2
   int c1, npiece, lr;           // rows per plane, pieces per row, log2 lanes
-  int dx, bx;                   // STR: units from one to the next in the dat (those of an
-                                // element) and the buffer (those of a point)
-  long long comp;               // STR: units from one component to the next in the dat
-  unsigned first;               // STR: box of blockIdx.y 0
+  int w, per;                   // SOA: units of an element, of a point in the buffer
+  long long comp;               // SOA: units from one component to the next in the dat
   int dir;                      // 0 dat -> buffer, 1 buffer -> dat
 };
 
-template <typename U, bool STR>
+template <typename U, bool SOA>
 __global__ void __launch_bounds__(256) box_copy_kernel(U *__restrict__ dat, U *__restrict__ buf,
                                                        const BoxRows g) {
   const int lane = threadIdx.x & ((1 << g.lr) - 1), ln = 1 << g.lr;
-  if (STR) {
-    const unsigned k = g.first + blockIdx.y;
-    dat += k / g.dx * g.comp + k % g.dx;
-    buf += k;
-  }
   const long long items = g.rows * g.npiece;
   const long long step = (long long)gridDim.x * (blockDim.x >> g.lr);
+  const int sx = SOA ? ln / g.per : 0, sk = SOA ? ln % g.per : 0;  // ln units on
   for (long long it = (long long)blockIdx.x * (blockDim.x >> g.lr) + (threadIdx.x >> g.lr);
        it < items; it += step) {
     long long row = it, z;
@@ -298,25 +291,43 @@ __global__ void __launch_bounds__(256) box_copy_kernel(U *__restrict__ dat, U *_
     U *d = dat + g.off + z * g.plane + y * g.pitch;
     U *b = buf + row * g.bstep;
     const long long end = g.npiece > 1 ? min(g.len, (long long)(piece + 1) * kPiece) : g.len;
-    long long x = (long long)piece * kPiece + lane;
-    const long long dx = STR ? g.dx : 1, bx = STR ? g.bx : 1;
+    long long e = (long long)piece * kPiece + lane;
+    // unit e of the row in the dat; SOA: unit k of point x
+    long long x = SOA ? (g.len >> 31 ? e / g.per : (long long)((unsigned)e / (unsigned)g.per)) : e;
+    int k = SOA ? (int)(e - x * g.per) : 0;
+    auto next = [&]() {
+      if (!SOA) {
+        const long long at = x;
+        x += ln;
+        return at;
+      }
+      const long long at = g.w == 1 ? x + k * g.comp : x * g.w + k / g.w * g.comp + k % g.w;
+      x += sx;
+      k += sk;
+      if (k >= g.per) {
+        k -= g.per;
+        x++;
+      }
+      return at;
+    };
     U v[4];
+    long long at[4];
     if (g.dir == 0) {
-      for (; x + 3 * ln < end; x += 4 * ln) {
+      for (; e + 3 * ln < end; e += 4 * ln) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) v[k] = d[(x + k * ln) * dx];
+        for (int j = 0; j < 4; j++) v[j] = d[next()];
 #pragma unroll
-        for (int k = 0; k < 4; k++) b[(x + k * ln) * bx] = v[k];
+        for (int j = 0; j < 4; j++) b[e + j * ln] = v[j];
       }
-      for (; x < end; x += ln) b[x * bx] = d[x * dx];
+      for (; e < end; e += ln) b[e] = d[next()];
     } else {
-      for (; x + 3 * ln < end; x += 4 * ln) {
+      for (; e + 3 * ln < end; e += 4 * ln) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) v[k] = b[(x + k * ln) * bx];
+        for (int j = 0; j < 4; j++) at[j] = next(), v[j] = b[e + j * ln];
 #pragma unroll
-        for (int k = 0; k < 4; k++) d[(x + k * ln) * dx] = v[k];
+        for (int j = 0; j < 4; j++) d[at[j]] = v[j];
       }
-      for (; x < end; x += ln) d[x * dx] = b[x * bx];
+      for (; e < end; e += ln) d[next()] = b[e];
     }
   }
 }
@@ -330,11 +341,7 @@ int launch_box(char *dat, char *buf, BoxRows g, bool apart) {
   const long long need = (g.rows * g.npiece + per - 1) / per;
   const unsigned blocks = (unsigned)std::min(need, 32LL * g_sms);
   if (apart)
-    for (int k = 0; k < g.bx; k += 65535) {
-      g.first = k;
-      box_copy_kernel<U, true><<<dim3(blocks, std::min(g.bx - k, 65535)), 256, 0, g_stream>>>(
-          (U *)dat, (U *)buf, g);
-    }
+    box_copy_kernel<U, true><<<blocks, 256, 0, g_stream>>>((U *)dat, (U *)buf, g);
   else
     box_copy_kernel<U, false><<<blocks, 256, 0, g_stream>>>((U *)dat, (U *)buf, g);
   return rc(cudaGetLastError());
@@ -362,9 +369,9 @@ OB2_API int ob2_box_copy(char *dat, int ts, int nc, int soa, const int *size3, c
   g.bstep = (long long)count3[0] * nc * w;
   g.c1 = count3[1];
   g.dir = dir;
-  g.len = apart ? count3[0] : count3[0] * m;
-  g.dx = apart ? w : 1;
-  g.bx = apart ? nc * w : 1;
+  g.len = g.bstep;
+  g.w = w;
+  g.per = nc * w;
   g.comp = sy * size3[2] * w;
   return u == 8   ? launch_box<unsigned long long>(dat, buf, g, apart)
          : u == 4 ? launch_box<unsigned int>(dat, buf, g, apart)
