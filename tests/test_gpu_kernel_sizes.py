@@ -28,6 +28,17 @@ def test_reduction_tiles(args):
     assert_lines_close(result_lines(gout), result_lines(cout), 1e-11)
 
 
+@pytest.mark.parametrize("n", [5, 70, 700])
+def test_reduction_results(n):
+    """Every way a result takes to the host (apps/redunit): the oracle's
+    lines, digit by digit (the sums are exact in any order)."""
+    gout, _ = run_app("redunit", "b200", ["-n=%d" % n])
+    cout, _ = run_app("redunit", "oracle", ["-n=%d" % n])
+    lines = [l for l in cout.splitlines() if l.startswith("sums")]
+    assert len(lines) == 17 + 3 + 3
+    assert [l for l in gout.splitlines() if l.startswith("sums")] == lines
+
+
 @pytest.mark.parametrize("name,args", [
     ("poisson_mb", ["-nb=1", "-n=1921", "-sweeps=2", "-check=1"]),
     ("poisson_mb", ["-nb=1", "-n=2048", "-sweeps=2", "-check=1"]),
