@@ -292,42 +292,38 @@ __global__ void __launch_bounds__(256) box_copy_kernel(U *__restrict__ dat, U *_
     U *b = buf + row * g.bstep;
     const long long end = g.npiece > 1 ? min(g.len, (long long)(piece + 1) * kPiece) : g.len;
     long long e = (long long)piece * kPiece + lane;
-    // unit e of the row in the dat; SOA: unit k of point x
-    long long x = SOA ? (g.len >> 31 ? e / g.per : (long long)((unsigned)e / (unsigned)g.per)) : e;
+    // SOA: unit e of the row is unit k of point x
+    long long x = SOA ? (g.len >> 31 ? e / g.per : (long long)((unsigned)e / (unsigned)g.per)) : 0;
     int k = SOA ? (int)(e - x * g.per) : 0;
-    auto next = [&]() {
-      if (!SOA) {
-        const long long at = x;
-        x += ln;
-        return at;
-      }
-      const long long at = g.w == 1 ? x + k * g.comp : x * g.w + k / g.w * g.comp + k % g.w;
+    // where unit e + j * ln lies in the dat's row (asked for in order)
+    auto at = [&](int j) {
+      if (!SOA) return e + j * ln;
+      const long long o = g.w == 1 ? x + k * g.comp : x * g.w + k / g.w * g.comp + k % g.w;
       x += sx;
       k += sk;
       if (k >= g.per) {
         k -= g.per;
         x++;
       }
-      return at;
+      return o;
     };
     U v[4];
-    long long at[4];
     if (g.dir == 0) {
       for (; e + 3 * ln < end; e += 4 * ln) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = d[next()];
+        for (int j = 0; j < 4; j++) v[j] = d[at(j)];
 #pragma unroll
         for (int j = 0; j < 4; j++) b[e + j * ln] = v[j];
       }
-      for (; e < end; e += ln) b[e] = d[next()];
+      for (; e < end; e += ln) b[e] = d[at(0)];
     } else {
       for (; e + 3 * ln < end; e += 4 * ln) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) at[j] = next(), v[j] = b[e + j * ln];
+        for (int j = 0; j < 4; j++) v[j] = b[e + j * ln];
 #pragma unroll
-        for (int j = 0; j < 4; j++) d[at[j]] = v[j];
+        for (int j = 0; j < 4; j++) d[at(j)] = v[j];
       }
-      for (; e < end; e += ln) d[next()] = b[e];
+      for (; e < end; e += ln) d[at(0)] = b[e];
     }
   }
 }
