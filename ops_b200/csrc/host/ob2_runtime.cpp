@@ -2507,6 +2507,13 @@ OPS_API int ob2_loop_begin(ob2_loop *L, const char *name, ops_block block, int d
         ex << "Error: reduction handle " << h->name << " used without ops_arg_reduce";
         throw ex;
       }
+      if (x.pending_first && (size_t)a.dim * type_bytes(type_code(h->type)) < (size_t)h->size) {
+        // the components that this loop does not feed start from the identity,
+        // too (h->data holds it since ops_arg_reduce)
+        memcpy(x.host_pinned, h->data, h->size);
+        check(ob2_dev_h2d_async(x.acc_d, x.host_pinned, h->size), "ops_arg_reduce");
+        x.pending_first = 0;
+      }
       L->red[i].acc = x.acc_d;
       L->red[i].first = x.pending_first;
       L->red[i].op = a.acc;
