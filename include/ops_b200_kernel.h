@@ -157,7 +157,7 @@ __device__ __forceinline__ void publish(const T &v, int d, unsigned long long *s
 }
 
 /* Step 3 (last CTA, every reduction argument): fixed-order combine of all
- * partials, folded into the handle's accumulator and published. */
+ * partials, folded into the handle's accumulator and, for a key, published. */
 template <typename T, int OP>
 __device__ __forceinline__ void final_combine(int dim, const T *part, T *acc, int first, T *sh,
                                               unsigned long long *slots, unsigned long long key) {
@@ -172,7 +172,7 @@ __device__ __forceinline__ void final_combine(int dim, const T *part, T *acc, in
     if (t == 0) {
       v = first ? v : combine<T, OP>(acc[d], v);
       acc[d] = v;
-      publish(v, d, slots, key);
+      if (key) publish(v, d, slots, key);
     }
   }
 }

@@ -36,7 +36,7 @@ typedef struct ob2_red {
   int first;    /* 1: this loop initialises the accumulator */
   int op;       /* OPS_INC / OPS_MIN / OPS_MAX */
   unsigned long long *slots;  /* the handle's pinned slots (ob2::publish) */
-  unsigned long long key;     /* this launch's key */
+  unsigned long long key;     /* this launch's key; 0: not published */
 } ob2_red;
 
 /* A generated fused launcher (one per application): runs n (<= OB2_FUSE_MAX)
