@@ -25,6 +25,8 @@ def ensure(name: str, flavour: str, shared: bool = True) -> str:
         return path
     if not catalog.available(name):
         pytest.skip("%s/%s not built and its sources are not present" % (name, flavour))
+    if flavour.startswith("ref_") and not (catalog.REF and os.path.isdir(catalog.REF)):
+        pytest.skip("%s/%s not built and the reference tree is not present" % (name, flavour))
     return catalog.build(name, flavour, shared=shared)
 
 
