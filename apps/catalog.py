@@ -61,6 +61,7 @@ APPS = {
     "opsunit": ("own", os.path.join(ROOT, "apps", "opsunit"), ["opsunit.cpp"], None),
     "hdunit": ("own", os.path.join(ROOT, "apps", "hdunit"), ["hdunit.cpp"], None),
     "redunit": ("own", os.path.join(ROOT, "apps", "redunit"), ["redunit.cpp"], None),
+    "sweep3d": ("own", os.path.join(ROOT, "apps", "sweep3d"), ["sweep3d.cpp"], None),
     "ref_poisson": ("ref", os.path.join(_REF_ROOT, "apps", "c", "poisson"), ["poisson.cpp"], None),
     "ref_mblock": ("ref", os.path.join(_REF_ROOT, "apps", "c", "mblock"), ["mblock.cpp"], None),
     # 4D blocks: two 4^4 blocks filled from ops_arg_idx, joined by a 4D halo

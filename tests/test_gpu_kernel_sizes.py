@@ -62,6 +62,23 @@ def test_common_layout_tiles(name, args):
             assert d <= (1e-5 if dat in ("x", "r32", "p32", "w32") else 1e-10), (dat, d)
 
 
+@pytest.mark.parametrize("args", [["-nx=131", "-ny=97", "-nz=151"],
+                                  ["-nx=160", "-ny=130", "-nz=100", "-off=1"],
+                                  ["-nx=33", "-ny=253", "-nz=239"],
+                                  ["-nx=9", "-ny=7", "-nz=5"]])
+def test_common_layout_rows_in_3d(args):
+    """3D loops with several rows per thread (apps/sweep3d: 2 in double, 4 in
+    float) over extents that are no multiple of a tile, through the kernels
+    for dats of one layout: dats and reductions as the oracle's, bit for
+    bit."""
+    gout, gd = run_app("sweep3d", "b200", args, dump=True)
+    cout, cd = run_app("sweep3d", "oracle", args, dump=True)
+    diffs = compare(gd, cd)
+    assert len(diffs) == 5 and max(diffs.values()) == 0.0, diffs
+    lines = [l for l in cout.splitlines() if l.startswith("max")]
+    assert lines and [l for l in gout.splitlines() if l.startswith("max")] == lines
+
+
 LINES = [2, 5, 40, 41, 48, 49, 64, 65, 80, 96, 97, 128, 129, 160, 161, 192, 193, 224, 225, 256,
          257, 511, 1537, 2048, 2049, 4096]
 
@@ -73,10 +90,11 @@ def test_trid_line_lengths(typ, solvedim, n):
     """Line lengths at the edges of the chunk (5 to 8 points), lane (8, 16,
     32) and segment (256 points, 2 to 16 of them) ranges, unit-stride and
     strided, with and without _Inc, against the numpy Thomas model
-    (test_trid_batch: 1e-12 relative, diagonally dominant systems)."""
+    (test_trid_batch: 1e-12 relative, diagonally dominant systems; it solves a
+    range of two points less than the shape along x and y)."""
     from tests.test_gpu_cabi import test_trid_batch
-    others = [9, 5] if n < 1000 else [9, 2]
-    shape = others[:solvedim] + [n] + others[solvedim:]
+    others = [9, 5] if n < 1000 else [9, 4 if solvedim == 0 else 2]
+    shape = others[:solvedim] + [n if solvedim == 2 else n + 2] + others[solvedim:]
     for inc in (False, True):
         test_trid_batch(typ, solvedim, inc, tuple(shape))
 
@@ -90,6 +108,50 @@ def test_trid_segments(typ, segments):
     from tests.test_gpu_cabi import test_trid_batch
     for inc in (False, True, False):
         test_trid_batch(typ, 1, inc, (7, 256 * segments - 35, 2))
+
+
+@pytest.mark.parametrize("typ", ["double", "float"])
+@pytest.mark.parametrize("n", [3, 61, 119, 250, 700, 2500])
+def test_trid_offsets_beyond_32_bits(typ, n):
+    """Strided lines whose elements lie more than 2^31 apart (the third axis
+    strides over 2^31 elements of one sparse buffer that holds every array),
+    with and without _Inc, starting at an odd element."""
+    import ctypes as C
+
+    import numpy as np
+    import torch
+
+    from tests import cabi
+    from tests.test_gpu_cabi import thomas
+    L = cabi.lib()
+    L.ob2_trid_batch.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int),
+                                 C.POINTER(C.c_longlong)] + [C.c_void_p] * 5
+    ts, dt = (8, torch.float64) if typ == "double" else (4, torch.float32)
+    far, apart, nx = 1 << 31, 1 << 20, 3
+    buf = torch.empty(far + 5 * apart, dtype=dt, device="cuda")
+    rng = np.random.default_rng(n)
+    vals = {k: rng.uniform(-1, 1, (2, n, nx)) + (4.0 if k == "b" else 0.0) for k in "abcdu"}
+    view = {k: buf[1 + j * apart:].as_strided((2, n, nx), (far, 7, 1)) for j, k in enumerate("abcdu")}
+    strides = (C.c_longlong * 3)(1, 7, far)
+    for inc in (False, True):
+        for k in "abcdu":
+            vals[k] = vals[k].astype(np.float64 if ts == 8 else np.float32)
+            view[k].copy_(torch.from_numpy(vals[k]))
+        torch.cuda.synchronize()
+        p = [view[k].data_ptr() for k in "abcd"] + [view["u"].data_ptr() if inc else None]
+        assert L.ob2_trid_batch(ts, 3, 1, cabi.ivec([nx, n, 2]), strides, *p) == 0
+        torch.cuda.synchronize()
+        got = view["u" if inc else "d"].cpu().numpy()
+        want = vals["u"].astype(np.float64) if inc else np.zeros((2, n, nx))
+        for z in range(2):
+            for x in range(nx):
+                want[z, :, x] += thomas(*(vals[k][z, :, x].astype(np.float64) for k in "abcd"))
+        if ts == 8:
+            np.testing.assert_allclose(got, want, rtol=1e-12, atol=1e-13)
+        else:  # one rounding to float, after u is added
+            np.testing.assert_allclose(got, want, rtol=2.5e-7, atol=1e-6)
+    del view, buf
+    torch.cuda.empty_cache()
 
 
 def test_trid_too_long_is_refused():
