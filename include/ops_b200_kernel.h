@@ -183,13 +183,29 @@ __device__ __forceinline__ void reset_counter(unsigned int *counter) {
   if (t == 0) *counter = 0u;
 }
 
-/* tile t of nt along x, then y, then z (32-bit division whenever nt fits) */
-__device__ __forceinline__ void tile_of(unsigned long long t, unsigned long long nt, unsigned tx,
-                                        unsigned ty, unsigned &bx, unsigned &by, unsigned &bz) {
-  unsigned long long r = nt >> 32 ? t / tx : (unsigned long long)((unsigned)t / tx);
-  bx = (unsigned)(t - r * tx);
-  bz = nt >> 32 ? (unsigned)(r / ty) : (unsigned)r / ty;
-  by = (unsigned)(r - (unsigned long long)bz * ty);
+/* tile t along x, then y, then z */
+__device__ __forceinline__ void tile_of(unsigned t, unsigned tx, unsigned ty, unsigned &bx,
+                                        unsigned &by, unsigned &bz) {
+  const unsigned r = t / tx;
+  bx = t - r * tx;
+  bz = r / ty;
+  by = r - bz * ty;
+}
+
+/* ... and the tile `s` further on (s < the tile counts in x and y) */
+__device__ __forceinline__ void tile_step(unsigned tx, unsigned ty, unsigned sx, unsigned sy,
+                                          unsigned sz, unsigned &bx, unsigned &by, unsigned &bz) {
+  bx += sx;
+  by += sy;
+  bz += sz;
+  if (bx >= tx) {
+    bx -= tx;
+    by++;
+  }
+  if (by >= ty) {
+    by -= ty;
+    bz++;
+  }
 }
 
 /* CTAs of `threads` threads of a kernel without dynamic shared memory that

@@ -198,8 +198,9 @@ OPS_API void ob2_loop_end(ob2_loop *L);
  * size do not fill half a wave of CTAs (`resident` per SM, times
  * OPS_B200_RED_WAVES).  tiles[0..2] = tiles of L->block along x (block[0] *
  * cols columns), y (block[1] * rows rows) and z (the folded 3rd to 5th axes).
- * Returns the CTAs: one wave at most, evened out over the trips; L->partials
- * is made large enough for them. */
+ * Under the default CTA shape L->block is fitted to thin ranges (as many
+ * threads, at most).  Returns the CTAs: one wave at most, evened out over the
+ * trips; L->partials is made large enough for them. */
 OPS_API unsigned ob2_red_grid(ob2_loop *L, int *cols, int *rows, int resident,
                               unsigned tiles[3]);
 /* 1 when some dat is passed more than once and written through one of the

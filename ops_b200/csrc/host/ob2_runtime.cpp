@@ -2572,11 +2572,25 @@ OPS_API unsigned ob2_red_grid(ob2_loop *L, int *cols, int *rows, int resident,
   // several columns per thread only in long rows: the tiles cut off at their
   // end are taken point by point (a CG's 1000 x 777 update: 11.1 us with 4
   // columns, 9.3 us with 1; 4096^2: 133 against 138 us)
+  const bool by32 = *cols > 1;  // the columns of a thread lie 32 apart
   if (L->n[0] < 16LL * L->block[0] * *cols) *cols = 1;
   // several points per thread only where the tiles still fill half the GPU (a
   // CG's 200 x 177 update: 4.7 us with 1 row, 6.9 us with 4; at 1000 x 777
   // 11.1 against 8.7 us)
   for (;; *cols = *rows = 1) {
+    // under the default shape no more threads along y and z than a thin range
+    // has rows for (sum over 4000 x 1 x 1000 points: 149 us with 32 x 8 x 1
+    // threads, 25 us with 32 x 1 x 8)
+    if (!r.block_set) {
+      auto cover = [](long long n, int most) {  // least power of two that holds n
+        int b = 1;
+        while (b < most && b < n) b *= 2;
+        return b;
+      };
+      L->block[1] = cover((ext[1] + *rows - 1) / *rows, 8);
+      L->block[2] = cover(ext[2], 8 / L->block[1]);
+      L->block[0] = by32 ? 32 : 256 / (L->block[1] * L->block[2]);
+    }
     const long long per[3] = {(long long)L->block[0] * *cols, (long long)L->block[1] * *rows,
                               L->block[2]};
     total = 1;

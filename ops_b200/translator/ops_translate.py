@@ -1142,8 +1142,9 @@ class Translator:
                 w("  %s *r%d; %s *part%d; int first%d;" % (p.base_type, i, p.base_type, i, i))
                 w("  unsigned long long *rs%d, rk%d;" % (i, i))
                 reds.append((i, a, p))
-        if reds:  # tiles along x, y and z; columns and rows per thread of a tile
-            w("  unsigned tx, ty, tz; int cols, rows;")
+        if reds:  # tiles along x, y and z, those a grid further on; columns and
+            # rows per thread of a tile
+            w("  unsigned tx, ty, tz, sx, sy, sz; int cols, rows;")
         w("};")
         # Point function, in two variants: with __restrict__ dat pointers
         # (the common case: no dat is both written and passed twice, so the
@@ -1265,9 +1266,12 @@ class Translator:
             # second wave; PY consecutive rows per thread and tile keep that
             # many rows' loads in flight
             w("  const unsigned long long nt = (unsigned long long)p.tx * p.ty * p.tz;")
-            w("  for (unsigned long long t = blockIdx.x; t < nt; t += gridDim.x) {")
-            w("    unsigned bx, by, bz;")
-            w("    ob2::tile_of(t, nt, p.tx, p.ty, bx, by, bz);")
+            # (a tile's coordinates by steps of the grid: divisions in every
+            # trip took as long as the loads of a range that fits L2)
+            w("  unsigned bx, by, bz;")
+            w("  ob2::tile_of(blockIdx.x, p.tx, p.ty, bx, by, bz);")
+            w("  for (unsigned long long t = blockIdx.x; t < nt; t += gridDim.x,"
+              " ob2::tile_step(p.tx, p.ty, p.sx, p.sy, p.sz, bx, by, bz)) {")
             w("    const int x = p.lo0 + (int)(bx * blockDim.x * p.cols + threadIdx.x);")
             w("    const int yb = p.lo1 + (int)(by * blockDim.y + threadIdx.y) * p.rows;")
             if hd:  # the 3rd to 5th axes as one folded index
@@ -1527,6 +1531,8 @@ class Translator:
             w("  grd = dim3(ob2_red_grid(&L, &p.cols, &p.rows, ob2::resident_ctas(kern, (int)"
               "(blk.x * blk.y * blk.z)), tiles), 1, 1);")
             w("  p.tx = tiles[0]; p.ty = tiles[1]; p.tz = tiles[2];")
+            w("  p.sx = grd.x % p.tx; p.sy = grd.x / p.tx % p.ty; p.sz = grd.x / p.tx / p.ty;")
+            w("  blk = dim3(L.block[0], L.block[1], L.block[2]);")
             w("  size_t nblk = (size_t)grd.x * grd.y * grd.z;")
             w("  char *scratch = (char *)L.partials;")
         for i, (a, p) in enumerate(zip(loop.args, kd.params)):

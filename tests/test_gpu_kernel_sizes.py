@@ -28,7 +28,7 @@ def test_reduction_tiles(args):
     assert_lines_close(result_lines(gout), result_lines(cout), 1e-11)
 
 
-@pytest.mark.parametrize("n", [5, 70, 700])
+@pytest.mark.parametrize("n", [5, 9, 20, 70, 700])
 def test_reduction_results(n):
     """Every way a result takes to the host (apps/redunit): the oracle's
     lines, digit by digit (the sums are exact in any order)."""
@@ -65,12 +65,14 @@ def test_common_layout_tiles(name, args):
 @pytest.mark.parametrize("args", [["-nx=131", "-ny=97", "-nz=151"],
                                   ["-nx=160", "-ny=130", "-nz=100", "-off=1"],
                                   ["-nx=33", "-ny=253", "-nz=239"],
-                                  ["-nx=9", "-ny=7", "-nz=5"]])
+                                  ["-nx=9", "-ny=7", "-nz=5"], ["-nx=1030", "-ny=2", "-nz=70"],
+                                  ["-nx=40", "-ny=3", "-nz=900"], ["-nx=3", "-ny=10", "-nz=901"],
+                                  ["-nx=257", "-ny=17", "-nz=3"], ["-nx=5000", "-ny=2", "-nz=2"]])
 def test_common_layout_rows_in_3d(args):
     """3D loops with several rows per thread (apps/sweep3d: 2 in double, 4 in
-    float) over extents that are no multiple of a tile, through the kernels
-    for dats of one layout: dats and reductions as the oracle's, bit for
-    bit."""
+    float) over extents that are no multiple of a tile, and thin ones, to which
+    the reduction's CTA shape is fitted, through the kernels for dats of one
+    layout: dats and reductions as the oracle's, bit for bit."""
     gout, gd = run_app("sweep3d", "b200", args, dump=True)
     cout, cd = run_app("sweep3d", "oracle", args, dump=True)
     diffs = compare(gd, cd)
