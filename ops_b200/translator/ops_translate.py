@@ -1507,10 +1507,15 @@ class Translator:
             # 1500^2 ran at 0.88 (FP64) and 0.73 (FP32) of the other kernel's
             # speed, 2048^2 at 1.12; half a wave without: p = r + b p of 1000 x
             # 777 3.7 against 4.8 us), and rows long enough that the tiles cut
-            # off at their end, taken point by point, are few
+            # off at their end, taken point by point, are few; with rows alone
+            # and little arithmetic, long enough for the warps (a stencil along
+            # y over 3 to 24 x 500 x 500 points: 20.3 against 17.5 us, 40 x 300
+            # x 300 13.9 against 13.5, equal from 64; with divisions 44.1
+            # against 47.6)
             big = " && L.npoints >= %dLL" % (148 * (3072 if pyu > 1 else 1024) * px * pyu) \
                 if not reds and px * pyu > py else ""
-            big += " && L.n[0] >= %d" % (128 * px) if not reds and px > 1 else ""
+            if not reds and px * pyu > 1 and (px > 1 or self.light_arithmetic(kd)):
+                big += " && L.n[0] >= %d" % (128 * px if px > 1 else 64)
             w("  const bool uni = !al && L.idx32%s%s &&\n    %s;" %
               (" && blk.x == 32" if px > 1 else "", big, " &&\n    ".join(cond)))
             if not reds and (px > 1 or pyu != py or (awu is None) != (aw is None)):
