@@ -110,10 +110,11 @@ __device__ __forceinline__ long long line_base(long long line, long long nlines,
 // A lane whose chunk lies inside the line loads and stores it with 16-byte
 // accesses, the line's partial last chunk element by element.
 //
-// Latency-bound (256^3 FP64: FP64 pipe 16 %, issue slots 28 % busy, 3 CTAs per
+// Latency-bound (256^3 FP64: FP64 pipe 18 %, issue slots 36 % busy, 3 CTAs per
 // SM by registers).  Measured: 256^3 167 us FP64 (161 before segments and
-// packed lines), 111 us FP32 (126); 2048 x 1500 44 us FP64 (109 with the PCR
-// of the whole line in shared memory), 36 us FP32 (84).
+// packed lines), 111 us FP32 (126); 300^3 269 us (715) and 246 us (537); 2048 x
+// 1500 44 us FP64 (109 with the PCR of the whole line in shared memory), 35 us
+// FP32 (83).
 template <typename T, bool INC, int SEG, int CL, int W>
 __global__ void __launch_bounds__(SEG == 2 ? 32 * kMaxSeg : kThreads, SEG == 2 ? 1 : 3) trid_x_kernel(
     int n, int S, long long nlines, int o1n, long long o1s, long long o2s, const T *__restrict__ A,
@@ -205,14 +206,18 @@ __global__ void __launch_bounds__(SEG == 2 ? 32 * kMaxSeg : kThreads, SEG == 2 ?
 // when every offset of the batch fits (IDX32).
 //
 // Bound by the latency of a CTA's load, elimination and PCR phases, three CTAs
-// per SM in different ones (256^3 y, FP64: 4.5 TB/s, FP64 pipe 18 %, issue
-// slots 39 % busy).  Measured, before: the same lines as 32 chunks of 8 rows
+// per SM in different ones (256^3 y, FP64: 4.5 TB/s, FP64 pipe 21 %, issue
+// slots 40 % busy).  The 80 registers of a thread that this takes do not hold
+// an 8-row chunk in FP64 whole: 6 values spill, 13 to 20 in the _Inc forms,
+// whose u is in flight during the PCR (z _Inc waits on memory 7 cycles per
+// issue, y 3).  Measured, before: the same lines as 32 chunks of 8 rows
 // whatever their length, lines over 256 points through shared-memory PCR.
-//   256^3       y FP64 147 -> 148 us, _Inc 234 -> 213; FP32 174 -> 101, 267 -> 133
-//               z FP64 203 -> 182 us, _Inc 263 -> 232; FP32 192 -> 131, 277 -> 162
+//   256^3       y FP64 146 -> 148 us, _Inc 234 -> 208; FP32 173 -> 100, 268 -> 134
+//               z FP64 201 -> 180 us, _Inc 262 -> 230; FP32 186 -> 122, 277 -> 160
 //   128^3       y FP64 33 -> 23 us, _Inc 57 -> 34
-//   193x131x67  z FP64 42 -> 25 us, _Inc 74 -> 37; FP32 68 -> 16, 103 -> 19
-//   2048x1500   y FP64 89 -> 45 us, _Inc 187 -> 60; FP32 103 -> 38, 224 -> 48
+//   193x131x67  z FP64 42 -> 25 us, _Inc 74 -> 33; FP32 68 -> 16, 103 -> 19
+//   2048x1500   y FP64 90 -> 47 us, _Inc 183 -> 62; FP32 100 -> 40, 218 -> 49
+//   1000x4096   y FP64 140 -> 78 us, _Inc 270 -> 103; FP32 154 -> 72, 345 -> 88
 template <typename T, bool INC, bool IDX32, bool SEG, int CL, int W>
 __global__ void __launch_bounds__(kThreads, CL > 8 ? 1 : 3) trid_s_kernel(
     int n, int S, long long nlines, long long stride, int o1n, long long o1s, long long o2s,

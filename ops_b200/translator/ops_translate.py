@@ -953,13 +953,24 @@ class Translator:
 
     def red_rows(self, dats) -> int:
         """Most consecutive rows per thread and tile of a reduction kernel:
-        4 when its dats read at most 24 bytes per point, so that a thread has
-        several rows' loads in flight, else 1 (the loads of one row are
-        enough, and more rows cost the registers that hold warps).  Measured
-        on one B200 at 4096^2, 1 / 2 / 4 / 8 rows: residual of a 5-point
-        stencil 80 / 63 / 59 / 60 us FP64 (16 B per point) and 79 / 60 / 46 /
-        42 us FP32, w = A p of a CG in FP32 (12 B) 98 / 94 / 71 / 77 us; the
-        FP64 residual with four dats (32 B) 138 / 150 / 166 / 167 us."""
+        4 when its dats read at most 32 bytes per point, so that a thread has
+        several rows' loads in flight, else 1.  Measured on one B200, 1 / 4
+        rows, the common-layout kernel and (in brackets) the general one:
+
+          reads  dats  loop                          1 row         4 rows
+           16 B   2    residual, 4096^2 FP64      90 (104) us    57 (58) us
+            8 B   2    ... FP32                   88 (93)        43 (49)
+           24 B   4    CG w = A p, 4096^2 FP64   104 (116)       94 (112)
+           12 B   4    ... FP32                  100 (110)       64 (72)
+           32 B   4    CG update, 4096^2 FP64    145 (146)      134 (140)
+           32 B   4    time step, 3840^2         161 (168)      147 (151)
+           24 B   6    CG residual, mixed        117 (128)      128 (153)
+           32 B   6    ... FP64                  145 (139)      153 (166)
+           32 B   6    ... FP64, 1000 x 777     11.9 (12.6)    10.4 (10.8)
+
+        The six-dat residuals lose with 4 rows on large grids (they run once
+        per solve) and gain on small ones; the bound in bytes does not tell
+        them from the four-dat loops."""
         if self.rpy:
             return self.rpy
         rd = sum(self.ELEM_BYTES.get(p.base_type, 8) for i, a, p in dats if a.acc != "OPS_WRITE")
